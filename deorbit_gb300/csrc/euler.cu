@@ -425,6 +425,7 @@ struct Grid {
     double* scratch = nullptr;  // pressure read-out
     double* ref_r0 = nullptr;   // hydrostatic reference (set_ref), allocated on first use
     double* ref_p0 = nullptr;
+    double* ref_pf = nullptr;   // its pressure at the z-faces
     double* ref_dp = nullptr;   // its well-balanced gravity face-pressure difference
     std::vector<void*> allocs;
     int64_t bytes = 0;
@@ -548,6 +549,14 @@ struct Grid {
         if (p.void_cons && p.ref_r0 && p.rho_cfl > 0) launches += 3;
     }
 
+    // What the Lop reads of the reference: face pressures, gravity source.
+    void form_ref() {
+        const int64_t nf = (int64_t)p.nx * p.ny * (p.nz + 1);
+        k_ref_pf<<<grid_of(nf), 256, 0, st>>>(p, ref_r0, ref_pf);
+        k_ref_dp<<<grid_of(p.n), 256, 0, st>>>(p, ref_pf, ref_dp);
+        launches += 2;
+    }
+
     void check_visc(const Ctl& c) {
         if (c.visc_err)
             throw SphError(SPH_ERR_STATE, "implicit viscosity: a grid-wide barrier wait ran out (device busy?)");
@@ -628,8 +637,12 @@ void to_params(deu::P& p, const eu_params& e) {
 // Weakest-flaw activation strain of grow_damage (hydro_cpu.cpp:254), formed
 // on the host with the host library's pow.
 void derive(deu::P& p) {
-    const deu::Mat& m = p.m;
-    p.mf = deu::mat_as<float>(m);
+    deu::Mat& m = p.m;
+    deu::mat_derive(m);
+    p.mf = deu::mat_f32(m);
+    p.d_dx = deu::div_by(p.dx);
+    p.d_3 = deu::div_by(3.0);
+    p.id2 = 1.0 / (p.dx * p.dx);
     p.eps_act = (m.Emod > 0 && m.wk > 0) ? std::pow(1.0 / (m.wk * p.dx * p.dx * p.dx), 1.0 / m.wm) : 0.0;
     p.invdx = 1.0 / p.dx;
     p.cf.y_i0 = (float)p.y_i0; p.cf.mu_i = (float)p.mu_i; p.cf.ymi = (float)(p.y_m - p.y_i0);
@@ -759,8 +772,7 @@ int eu_set_material(eu_grid* h, const sph_material* m) {
         derive(g->p);
         if (g->p.ref_r0) {  // the gravity source's reference pressures follow the material
             deu::DeviceScope ds(g->device);
-            deu::k_ref_dp<<<g->grid_of(g->p.n), 256, 0, g->st>>>(g->p, g->ref_r0, g->ref_dp);
-            g->launches++;
+            g->form_ref();
             g->check();
             EU_CUDA(cudaStreamSynchronize(g->st));
         }
@@ -789,15 +801,17 @@ int eu_set_ref(eu_grid* h) {
             g->ref_r0 = g->alloc(g->p.n);
             g->ref_p0 = g->alloc(g->p.n);
             g->ref_dp = g->alloc(g->p.n);
+            g->ref_pf = g->alloc((int64_t)g->p.nx * g->p.ny * (g->p.nz + 1));
         }
         deu::k_set_ref<<<g->grid_of(g->p.n), 256, 0, g->st>>>(g->p, g->g, g->ref_r0, g->ref_p0);
-        deu::k_ref_dp<<<g->grid_of(g->p.n), 256, 0, g->st>>>(g->p, g->ref_r0, g->ref_dp);
-        g->launches += 2;
+        g->launches++;
+        g->form_ref();
         g->check();
         EU_CUDA(cudaStreamSynchronize(g->st));
         g->p.ref_r0 = g->ref_r0;
         g->p.ref_p0 = g->ref_p0;
         g->p.ref_dp = g->ref_dp;
+        g->p.ref_pf = g->ref_pf;
         g->graph_valid = false;
     });
 }
@@ -810,6 +824,7 @@ int eu_clear_ref(eu_grid* h) {
         g->p.ref_r0 = nullptr;
         g->p.ref_p0 = nullptr;
         g->p.ref_dp = nullptr;
+        g->p.ref_pf = nullptr;
         g->graph_valid = false;
     });
 }
@@ -925,7 +940,7 @@ int eu_update_af(eu_grid* h, double dt) {
         if (!std::isfinite(dt)) throw SphError(SPH_ERR_ARG, "dt must be finite");
         deu::DeviceScope ds(g->device);
         if (g->p.c_act > 0 && g->p.tdec > 0) {  // update_af returns at once otherwise (hydro_cpu.cpp:391)
-            deu::k_set_step<<<1, 1, 0, g->st>>>(g->ctl, dt);
+            deu::k_set_step<<<1, 1, 0, g->st>>>(g->p, g->ctl, dt);
             deu::k_update_af<<<g->grid_of(g->p.n), 256, 0, g->st>>>(g->p, g->g, g->ctl);
             g->launches += 2;
         }
@@ -968,7 +983,7 @@ int eu_step(eu_grid* h, double dt) {
         deu::Grid* g = G(h);
         if (!(dt >= 0) || !std::isfinite(dt)) throw SphError(SPH_ERR_ARG, "dt must be finite and >= 0");
         deu::DeviceScope ds(g->device);
-        deu::k_set_step<<<1, 1, 0, g->st>>>(g->ctl, dt);
+        deu::k_set_step<<<1, 1, 0, g->st>>>(g->p, g->ctl, dt);
         g->launches++;
         g->enqueue_step(false);
         g->check();
@@ -1001,7 +1016,7 @@ int eu_implicit_visc(eu_grid* h, double dt) {
         if (!(dt >= 0) || !std::isfinite(dt)) throw SphError(SPH_ERR_ARG, "dt must be finite and >= 0");
         deu::DeviceScope ds(g->device);
         if (g->visc_on()) {  // implicit_visc returns at once otherwise (hydro_cpu.cpp:302)
-            deu::k_set_step<<<1, 1, 0, g->st>>>(g->ctl, dt);
+            deu::k_set_step<<<1, 1, 0, g->st>>>(g->p, g->ctl, dt);
             g->launches++;
             g->enqueue_visc();
         }

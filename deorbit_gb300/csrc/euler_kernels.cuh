@@ -16,7 +16,56 @@
 
 #include <cstdint>
 
+#include "fp64_int.cuh"
+
 namespace deu {
+
+// ---------------------------------------------------------------- arithmetic by compute type
+
+// Divisions, square roots, comparisons and halvings in the compute type R: FP32
+// as written; FP64 with the same IEEE results from the integer pipes
+// (fp64_int.cuh), because the FP64 kernels here wait on the FP64 pipe and
+// nothing else.  On the 96^3 impact (ncu) a face flux was 671 FP64
+// instructions and is 195 with these, the EOS's shared subexpressions and one
+// HLLC side per face; a face pass 1.14 -> 0.35 ms, a right-hand side 865 -> 266
+// instructions and 1.46 -> 0.61 ms, the step 11.1 -> 4.0 ms, same bits.
+template <class R>
+struct DivBy;  // a divisor used more than once
+template <>
+struct DivBy<float> {
+    float b;
+};
+template <>
+struct DivBy<double> {
+    fi::Divisor d;
+};
+FI_FN DivBy<float> div_by(float b) { return DivBy<float>{b}; }
+FI_FN DivBy<double> div_by(double b) { return DivBy<double>{fi::divisor(b)}; }
+FI_FN float dv(float a, const DivBy<float>& d) { return a / d.b; }
+FI_FN double dv(double a, const DivBy<double>& d) { return fi::div(a, d.d); }
+FI_FN float dv(float a, float b) { return a / b; }
+FI_FN double dv(double a, double b) { return fi::div(a, b); }
+static __device__ __forceinline__ float root(float x) { return sqrtf(x); }
+static __device__ __forceinline__ double root(double x) { return fi::sqrt(x); }
+FI_FN float half(float x) { return 0.5f * x; }
+FI_FN double half(double x) { return fi::half(x); }
+FI_FN bool lt(float a, float b) { return a < b; }
+FI_FN bool lt(double a, double b) { return fi::lt(a, b); }
+FI_FN bool ge(float a, float b) { return a >= b; }
+FI_FN bool ge(double a, double b) { return fi::le(b, a); }
+FI_FN bool lt0(float x) { return x < 0.0f; }
+FI_FN bool lt0(double x) { return fi::lt0(x); }
+FI_FN bool gt0(float x) { return x > 0.0f; }
+FI_FN bool gt0(double x) { return fi::gt0(x); }
+FI_FN bool ge0(float x) { return x >= 0.0f; }
+FI_FN bool ge0(double x) { return fi::ge0(x); }
+FI_FN bool le0(float x) { return x <= 0.0f; }
+FI_FN bool le0(double x) { return fi::le0(x); }
+// a + m / 2: the halving is exact, so one fused operation rounds as the two do
+static __device__ __forceinline__ float add_half(float a, float m) { return a + 0.5f * m; }
+static __device__ __forceinline__ double add_half(double a, double m) { return __fma_rn(0.5, m, a); }
+static __device__ __forceinline__ float sub_half(float a, float m) { return a - 0.5f * m; }
+static __device__ __forceinline__ double sub_half(double a, double m) { return __fma_rn(-0.5, m, a); }
 
 // ---------------------------------------------------------------- materials
 
@@ -24,13 +73,27 @@ template <class R>
 struct MatT {
     int32_t ideal;
     R gamma, rho0, a, b, A, B, alpha, beta, u0, uiv, ucv, G, Y, Emod, wm, wk;
+    // formed once on the host (mat_derive): quotients and divisors of the constants above
+    R A_rho0, B2, iuv;
+    DivBy<R> d_rho0, d_uv, d_Emod;
 };
 using Mat = MatT<double>;
 
 template <class R>
-__host__ __device__ __forceinline__ MatT<R> mat_as(const Mat& m) {
-    return MatT<R>{m.ideal, R(m.gamma), R(m.rho0), R(m.a), R(m.b), R(m.A), R(m.B), R(m.alpha), R(m.beta),
-                   R(m.u0), R(m.uiv), R(m.ucv), R(m.G), R(m.Y), R(m.Emod), R(m.wm), R(m.wk)};
+inline void mat_derive(MatT<R>& m) {
+    m.A_rho0 = m.A / m.rho0;
+    m.B2 = R(2) * m.B;
+    m.iuv = R(1) / (m.ucv - m.uiv);
+    m.d_rho0 = div_by(m.rho0);
+    m.d_uv = div_by(m.ucv - m.uiv);
+    m.d_Emod = div_by(m.Emod);
+}
+inline MatT<float> mat_f32(const Mat& m) {
+    MatT<float> f{m.ideal, float(m.gamma), float(m.rho0), float(m.a), float(m.b), float(m.A), float(m.B),
+                  float(m.alpha), float(m.beta), float(m.u0), float(m.uiv), float(m.ucv), float(m.G), float(m.Y),
+                  float(m.Emod), float(m.wm), float(m.wk)};
+    mat_derive(f);
+    return f;
 }
 
 // Settings + material + grid geometry, passed by value to every kernel.
@@ -46,12 +109,14 @@ struct P {
     int32_t axisym, rock, af_reg, af_prel, af_seeddp;
     int32_t nx, ny, nz;
     int64_t n;
-    double dx, invdx;
+    double dx, invdx, id2;  // cell width, 1 / dx, 1 / dx^2
+    DivBy<double> d_dx, d_3;  // divisors dx and 3
     double eps_act;  // weakest-flaw activation strain, formed on the host as in hydro_cpu.cpp:254
     // hydrostatic reference of set_ref (hydro_cpu.cpp:259-261), null when off:
     // the well-balanced z-sweep and gravity source and the void-cell reset
     const double* ref_r0;
     const double* ref_p0;
+    const double* ref_pf;  // reference pressure at every z-face (zero internal energy, clamped at 0)
     const double* ref_dp;  // per cell p0(top face) - p0(bottom face) of the well-balanced gravity source
     double void_amb;  // VOID_AMB: void cells reset to this density instead of the reference's
     int32_t void_cons;  // VOID_CONS: the reset moves the excess mass to a neighbour first
@@ -81,89 +146,160 @@ __device__ __forceinline__ R narrow(double x) {
 __device__ __forceinline__ double widen(float y) { return (double)y; }
 __device__ __forceinline__ double widen(double y) { return y; }
 
-template <class R> __device__ __forceinline__ R dmax2(R a, R b) { return a < b ? b : a; }  // std::max
-template <class R> __device__ __forceinline__ R dmin2(R a, R b) { return b < a ? b : a; }  // std::min
+template <class R> __device__ __forceinline__ R dmax2(R a, R b) { return lt(a, b) ? b : a; }  // std::max
+template <class R> __device__ __forceinline__ R dmin2(R a, R b) { return lt(b, a) ? b : a; }  // std::min
+
+// The FP32 form's equation of state.
 
 // Tillotson pressure, eos.hpp:52-63.
-template <class R>
-__device__ R till(const MatT<R>& m, R rho, R u) {
-    if (rho <= R(0)) return R(0);
-    R eta = rho / m.rho0, mu = eta - R(1);
-    R w0 = u / (m.u0 * eta * eta) + R(1);
-    R Pc = (m.a + m.b / w0) * rho * u + m.A * mu + m.B * mu * mu;
+static __device__ float till(const MatT<float>& m, float rho, float u) {
+    if (rho <= 0.0f) return 0.0f;
+    float eta = rho / m.rho0, mu = eta - 1.0f;
+    float w0 = u / (m.u0 * eta * eta) + 1.0f;
+    float Pc = (m.a + m.b / w0) * rho * u + m.A * mu + m.B * mu * mu;
     if (rho >= m.rho0 || u <= m.uiv) return Pc;
-    R z = m.rho0 / rho - R(1);
-    R Pe = m.a * rho * u + (m.b * rho * u / w0 + m.A * mu * exp(-m.beta * z)) * exp(-m.alpha * z * z);
+    float z = m.rho0 / rho - 1.0f;
+    float Pe = m.a * rho * u + (m.b * rho * u / w0 + m.A * mu * exp(-m.beta * z)) * exp(-m.alpha * z * z);
     if (u >= m.ucv) return Pe;
     return ((u - m.uiv) * Pe + (m.ucv - u) * Pc) / (m.ucv - m.uiv);
 }
 
-template <class R>
-__device__ __forceinline__ R pressure(const MatT<R>& m, R rho, R u) {  // eos.hpp:65-68
-    if (m.ideal) return (m.gamma - R(1)) * rho * u;
+static __device__ __forceinline__ float pressure(const MatT<float>& m, float rho, float u) {  // eos.hpp:65-68
+    if (m.ideal) return (m.gamma - 1.0f) * rho * u;
     return till(m, rho, u);
 }
 
 // Condensed-branch value and analytic derivatives, eos.hpp:72-79.
-template <class R>
-__device__ void cond_d(const MatT<R>& m, R rho, R u, R& P, R& dPdr, R& dPdu) {
-    R eta = rho / m.rho0, mu = eta - R(1);
-    R w = R(1) + u / (m.u0 * eta * eta), aob = m.a + m.b / w;
+static __device__ void cond_d(const MatT<float>& m, float rho, float u, float& P, float& dPdr, float& dPdu) {
+    float eta = rho / m.rho0, mu = eta - 1.0f;
+    float w = 1.0f + u / (m.u0 * eta * eta), aob = m.a + m.b / w;
     P = aob * rho * u + m.A * mu + m.B * mu * mu;
     dPdu = aob * rho - m.b * rho * u / (w * w * m.u0 * eta * eta);
-    R dwdr = R(-2) * u / (m.u0 * eta * eta * eta * m.rho0);
-    dPdr = aob * u + rho * u * (-m.b / (w * w)) * dwdr + m.A / m.rho0 + R(2) * m.B * mu / m.rho0;
+    float dwdr = -2.0f * u / (m.u0 * eta * eta * eta * m.rho0);
+    dPdr = aob * u + rho * u * (-m.b / (w * w)) * dwdr + m.A / m.rho0 + 2.0f * m.B * mu / m.rho0;
 }
 
 // Expanded-branch value and analytic derivatives, eos.hpp:80-94.
-template <class R>
-__device__ void expd_d(const MatT<R>& m, R rho, R u, R& P, R& dPdr, R& dPdu) {
-    R eta = rho / m.rho0, mu = eta - R(1);
-    R w = R(1) + u / (m.u0 * eta * eta);
-    R z = m.rho0 / rho - R(1), dzdr = -m.rho0 / (rho * rho);
-    R E1 = exp(-m.alpha * z * z), E2 = exp(-m.beta * z);
-    R G = m.b * rho * u / w + m.A * mu * E2;
+static __device__ void expd_d(const MatT<float>& m, float rho, float u, float& P, float& dPdr, float& dPdu) {
+    float eta = rho / m.rho0, mu = eta - 1.0f;
+    float w = 1.0f + u / (m.u0 * eta * eta);
+    float z = m.rho0 / rho - 1.0f, dzdr = -m.rho0 / (rho * rho);
+    float E1 = exp(-m.alpha * z * z), E2 = exp(-m.beta * z);
+    float G = m.b * rho * u / w + m.A * mu * E2;
     P = m.a * rho * u + G * E1;
-    R dwdr = R(-2) * u / (m.u0 * eta * eta * eta * m.rho0);
-    R dGu = m.b * rho / w - m.b * rho * u / (w * w * m.u0 * eta * eta);
+    float dwdr = -2.0f * u / (m.u0 * eta * eta * eta * m.rho0);
+    float dGu = m.b * rho / w - m.b * rho * u / (w * w * m.u0 * eta * eta);
     dPdu = m.a * rho + dGu * E1;
-    R dbruw_dr = m.b * u / w + m.b * rho * u * (R(-1) / (w * w)) * dwdr;
-    R dGr = dbruw_dr + m.A * E2 / m.rho0 + m.A * mu * (E2 * (-m.beta) * dzdr);
-    R dE1dr = E1 * (-m.alpha * R(2) * z) * dzdr;
+    float dbruw_dr = m.b * u / w + m.b * rho * u * (-1.0f / (w * w)) * dwdr;
+    float dGr = dbruw_dr + m.A * E2 / m.rho0 + m.A * mu * (E2 * (-m.beta) * dzdr);
+    float dE1dr = E1 * (-m.alpha * 2.0f * z) * dzdr;
     dPdr = m.a * u + dGr * E1 + G * dE1dr;
 }
 
 // Analytic sound speed, eos.hpp:95-113.
-template <class R>
-__device__ R sound_speed(const MatT<R>& m, R rho, R u) {
+static __device__ float sound_speed(const MatT<float>& m, float rho, float u) {
     if (m.ideal) {
-        R Pi = (m.gamma - R(1)) * rho * u;
-        return sqrt(dmax2(m.gamma * Pi / dmax2(rho, R(1e-30)), R(1e-12)));
+        float Pi = (m.gamma - 1.0f) * rho * u;
+        return sqrt(dmax2(m.gamma * Pi / dmax2(rho, 1e-30f), 1e-12f));
     }
-    if (rho <= R(0)) return R(1e-3);
-    R Pp, dPdr, dPdu;
+    if (rho <= 0.0f) return 1e-3f;
+    float Pp, dPdr, dPdu;
     if (rho >= m.rho0 || u <= m.uiv) {
         cond_d(m, rho, u, Pp, dPdr, dPdu);
     } else if (u >= m.ucv) {
         expd_d(m, rho, u, Pp, dPdr, dPdu);
     } else {
-        R Pc, dPcr, dPcu, Pe, dPer, dPeu;
+        float Pc, dPcr, dPcu, Pe, dPer, dPeu;
         cond_d(m, rho, u, Pc, dPcr, dPcu);
         expd_d(m, rho, u, Pe, dPer, dPeu);
-        R inv = R(1) / (m.ucv - m.uiv);
+        float inv = 1.0f / (m.ucv - m.uiv);
         Pp = ((u - m.uiv) * Pe + (m.ucv - u) * Pc) * inv;
         dPdu = ((Pe + (u - m.uiv) * dPeu) + (-Pc + (m.ucv - u) * dPcu)) * inv;
         dPdr = ((u - m.uiv) * dPer + (m.ucv - u) * dPcr) * inv;
     }
-    return sqrt(dmax2(dPdr + Pp / (rho * rho) * dPdu, R(1e-6)));
+    return sqrt(dmax2(dPdr + Pp / (rho * rho) * dPdu, 1e-6f));
 }
 
 // hydro_cpu.cpp:38: pressure clamped at 0 and the sound speed.
-template <class R>
-__device__ __forceinline__ void eos_pc(const MatT<R>& m, R rho, R e, R& p, R& cs) {
+static __device__ __forceinline__ void eos_pc(const MatT<float>& m, float rho, float e, float& p, float& cs) {
     p = pressure(m, rho, e);
-    if (p < R(0)) p = R(0);
+    if (p < 0.0f) p = 0.0f;
     cs = sound_speed(m, rho, e);
+}
+
+// The FP64 form's: the same expressions, each operation the reference's.
+
+// Tillotson pressure, eos.hpp:52-63.
+static __device__ double till(const MatT<double>& m, double rho, double u) {
+    if (le0(rho)) return 0.0;
+    double eta = dv(rho, m.d_rho0), mu = eta - 1.0;
+    double w0 = dv(u, m.u0 * eta * eta) + 1.0;
+    double Pc = (m.a + dv(m.b, w0)) * rho * u + m.A * mu + m.B * mu * mu;
+    if (ge(rho, m.rho0) || ge(m.uiv, u)) return Pc;
+    double z = dv(m.rho0, rho) - 1.0;
+    double Pe = m.a * rho * u + (dv(m.b * rho * u, w0) + m.A * mu * exp(-m.beta * z)) * exp(-m.alpha * z * z);
+    if (ge(u, m.ucv)) return Pe;
+    return dv((u - m.uiv) * Pe + (m.ucv - u) * Pc, m.d_uv);
+}
+
+static __device__ __forceinline__ double pressure(const MatT<double>& m, double rho, double u) {  // eos.hpp:65-68
+    if (m.ideal) return (m.gamma - 1.0) * rho * u;
+    return till(m, rho, u);
+}
+
+// hydro_cpu.cpp:38: pressure clamped at 0 and the sound speed, in one pass:
+// Tillotson pressure (eos.hpp:52-63), the condensed and expanded branches'
+// values and analytic derivatives (72-94) and the sound speed (95-113) share
+// their subexpressions, each formed by the reference's operations.
+static __device__ void eos_pc(const MatT<double>& m, double rho, double u, double& p, double& cs) {
+    if (m.ideal) {
+        const double Pi = (m.gamma - 1.0) * rho * u;
+        cs = root(dmax2(dv(m.gamma * Pi, dmax2(rho, 1e-30)), 1e-12));
+        p = lt0(Pi) ? 0.0 : Pi;
+        return;
+    }
+    if (le0(rho)) {
+        p = 0.0;
+        cs = 1e-3;
+        return;
+    }
+    const double eta = dv(rho, m.d_rho0), mu = eta - 1.0;
+    const double ue2 = m.u0 * eta * eta;
+    const double w = dv(u, ue2) + 1.0, aob = m.a + dv(m.b, w), ar = aob * rho;
+    const double Pc = ar * u + m.A * mu + m.B * mu * mu;
+    const double bru = m.b * rho * u, ww = w * w;
+    const double bt = dv(bru, ww * m.u0 * eta * eta);
+    const double dwdr = dv(-2.0 * u, ue2 * eta * m.rho0);
+    const double Cu = ar - bt;
+    const double Cr = aob * u + rho * u * dv(-m.b, ww) * dwdr + m.A_rho0 + dv(m.B2 * mu, m.d_rho0);
+    double P, Pp, dPdr, dPdu;  // P as eos.hpp:52-63 gives it, Pp as the sound speed's own value
+    if (ge(rho, m.rho0) || ge(m.uiv, u)) {
+        P = Pp = Pc;
+        dPdr = Cr;
+        dPdu = Cu;
+    } else {
+        const double z = dv(m.rho0, rho) - 1.0, dzdr = dv(-m.rho0, rho * rho);
+        const double E1 = exp(-m.alpha * z * z), E2 = exp(-m.beta * z);
+        const double G = dv(bru, w) + m.A * mu * E2;
+        const double Pe = m.a * rho * u + G * E1;
+        const double Eu = m.a * rho + (dv(m.b * rho, w) - bt) * E1;
+        const double dbruw_dr = dv(m.b * u, w) + bru * dv(-1.0, ww) * dwdr;
+        const double dGr = dbruw_dr + dv(m.A * E2, m.d_rho0) + m.A * mu * (E2 * (-m.beta) * dzdr);
+        const double Er = m.a * u + dGr * E1 + G * (E1 * (-m.alpha * 2.0 * z) * dzdr);
+        if (ge(u, m.ucv)) {
+            P = Pp = Pe;
+            dPdr = Er;
+            dPdu = Eu;
+        } else {
+            const double x = (u - m.uiv) * Pe + (m.ucv - u) * Pc;
+            P = dv(x, m.d_uv);
+            Pp = x * m.iuv;
+            dPdu = ((Pe + (u - m.uiv) * Eu) + (-Pc + (m.ucv - u) * Cu)) * m.iuv;
+            dPdr = ((u - m.uiv) * Er + (m.ucv - u) * Cr) * m.iuv;
+        }
+    }
+    cs = root(dmax2(dPdr + dv(Pp, rho * rho) * dPdu, 1e-6));
+    p = lt0(P) ? 0.0 : P;
 }
 
 // ---------------------------------------------------------------- face flux
@@ -178,80 +314,148 @@ __device__ __forceinline__ F5<R> flux_of(R r, R vn, R t1, R t2, R p, R E) {
     return F5<R>{r * vn, r * vn * vn + p, r * vn * t1, r * vn * t2, (E + p) * vn};
 }
 
+// FP32 fluxes.
+
 // Exact rarefaction into vacuum sampled at the face, hydro_cpu.cpp:43-53.
-template <class R>
-__device__ F5<R> vac_flux(const MatT<R>& m, R rM, R vnM, R t1M, R t2M, R eM, int side) {
-    R pM, cM;
+static __device__ F5<float> vac_flux(const MatT<float>& m, float rM, float vnM, float t1M, float t2M, float eM, int side) {
+    float pM, cM;
     eos_pc(m, rM, eM, pM, cM);
-    R g = rM * cM * cM / dmax2(pM, R(1e-30));
-    if (g < R(1.01)) g = R(1.01);
-    if (g > R(1e5)) g = R(1e5);
-    R s = (R)side, vn = s * vnM;
-    if (vn - cM >= R(0)) {
-        R E = rM * eM + R(0.5) * rM * (vnM * vnM + t1M * t1M + t2M * t2M);
-        return F5<R>{rM * vnM, rM * vnM * vnM + pM, rM * vnM * t1M, rM * vnM * t2M, (E + pM) * vnM};
+    float g = rM * cM * cM / dmax2(pM, 1e-30f);
+    if (g < 1.01f) g = 1.01f;
+    if (g > 1e5f) g = 1e5f;
+    float s = (float)side, vn = s * vnM;
+    if (vn - cM >= 0.0f) {
+        float E = rM * eM + 0.5f * rM * (vnM * vnM + t1M * t1M + t2M * t2M);
+        return F5<float>{rM * vnM, rM * vnM * vnM + pM, rM * vnM * t1M, rM * vnM * t2M, (E + pM) * vnM};
     }
-    if (vn + R(2) * cM / (g - R(1)) <= R(0)) return F5<R>{R(0), R(0), R(0), R(0), R(0)};
-    R u0 = R(2) / (g + R(1)) * (cM + R(0.5) * (g - R(1)) * vn), c0 = u0;
-    R r0 = rM * pow(c0 / cM, R(2) / (g - R(1))), p0 = pM * pow(r0 / rM, g), e0 = p0 / ((g - R(1)) * r0),
+    if (vn + 2.0f * cM / (g - 1.0f) <= 0.0f) return F5<float>{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float u0 = 2.0f / (g + 1.0f) * (cM + 0.5f * (g - 1.0f) * vn), c0 = u0;
+    float r0 = rM * pow(c0 / cM, 2.0f / (g - 1.0f)), p0 = pM * pow(r0 / rM, g), e0 = p0 / ((g - 1.0f) * r0),
       un0 = s * u0;
-    R E0 = r0 * e0 + R(0.5) * r0 * (un0 * un0 + t1M * t1M + t2M * t2M);
-    return F5<R>{r0 * un0, r0 * un0 * un0 + p0, r0 * un0 * t1M, r0 * un0 * t2M, (E0 + p0) * un0};
+    float E0 = r0 * e0 + 0.5f * r0 * (un0 * un0 + t1M * t1M + t2M * t2M);
+    return F5<float>{r0 * un0, r0 * un0 * un0 + p0, r0 * un0 * t1M, r0 * un0 * t2M, (E0 + p0) * un0};
 }
 
-template <class R>
-__device__ __forceinline__ F5<R> hllc_star(R r, R vn, R t1, R t2, R p, R E, R S, R Ss, F5<R> Fk) {
-    R f = r * (S - vn) / (S - Ss);
-    F5<R> Us{f, f * Ss, f * t1, f * t2, f * (E / r + (Ss - vn) * (Ss + p / (r * (S - vn))))};
-    F5<R> U{r, r * vn, r * t1, r * t2, E};
-    return F5<R>{Fk.r + S * (Us.r - U.r), Fk.mn + S * (Us.mn - U.mn), Fk.mt1 + S * (Us.mt1 - U.mt1),
+static __device__ __forceinline__ F5<float> hllc_star(float r, float vn, float t1, float t2, float p, float E, float S, float Ss, F5<float> Fk) {
+    float f = r * (S - vn) / (S - Ss);
+    F5<float> Us{f, f * Ss, f * t1, f * t2, f * (E / r + (Ss - vn) * (Ss + p / (r * (S - vn))))};
+    F5<float> U{r, r * vn, r * t1, r * t2, E};
+    return F5<float>{Fk.r + S * (Us.r - U.r), Fk.mn + S * (Us.mn - U.mn), Fk.mt1 + S * (Us.mt1 - U.mt1),
                  Fk.mt2 + S * (Us.mt2 - U.mt2), Fk.E + S * (Us.E - U.E)};
 }
 
 // HLLC, hydro_cpu.cpp:54-74.
-template <class R>
-__device__ F5<R> hllc(const MatT<R>& m, R rho_vac, R rL, R vnL, R t1L, R t2L, R eL, R rR, R vnR, R t1R, R t2R,
-                      R eR) {
-    if (rho_vac > R(0)) {
+static __device__ F5<float> hllc(const MatT<float>& m, float rho_vac, float rL, float vnL, float t1L, float t2L, float eL, float rR, float vnR, float t1R, float t2R,
+                      float eR) {
+    if (rho_vac > 0.0f) {
         bool vL = rL < rho_vac, vR = rR < rho_vac;
-        if (vL && vR) return F5<R>{R(0), R(0), R(0), R(0), R(0)};
+        if (vL && vR) return F5<float>{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         if (vR) return vac_flux(m, rL, vnL, t1L, t2L, eL, +1);
         if (vL) return vac_flux(m, rR, vnR, t1R, t2R, eR, -1);
     }
-    R pL, cL, pR, cR;
+    float pL, cL, pR, cR;
     eos_pc(m, rL, eL, pL, cL);
     eos_pc(m, rR, eR, pR, cR);
-    R SL = dmin2(vnL - cL, vnR - cR), SR = dmax2(vnL + cL, vnR + cR);
-    R Ss = (pR - pL + rL * vnL * (SL - vnL) - rR * vnR * (SR - vnR)) / (rL * (SL - vnL) - rR * (SR - vnR));
-    R EL = rL * eL + R(0.5) * rL * (vnL * vnL + t1L * t1L + t2L * t2L),
-      ER = rR * eR + R(0.5) * rR * (vnR * vnR + t1R * t1R + t2R * t2R);
-    if (SL >= R(0)) return flux_of(rL, vnL, t1L, t2L, pL, EL);
-    if (SR <= R(0)) return flux_of(rR, vnR, t1R, t2R, pR, ER);
-    if (Ss >= R(0)) return hllc_star(rL, vnL, t1L, t2L, pL, EL, SL, Ss, flux_of(rL, vnL, t1L, t2L, pL, EL));
+    float SL = dmin2(vnL - cL, vnR - cR), SR = dmax2(vnL + cL, vnR + cR);
+    float Ss = (pR - pL + rL * vnL * (SL - vnL) - rR * vnR * (SR - vnR)) / (rL * (SL - vnL) - rR * (SR - vnR));
+    float EL = rL * eL + 0.5f * rL * (vnL * vnL + t1L * t1L + t2L * t2L),
+      ER = rR * eR + 0.5f * rR * (vnR * vnR + t1R * t1R + t2R * t2R);
+    if (SL >= 0.0f) return flux_of(rL, vnL, t1L, t2L, pL, EL);
+    if (SR <= 0.0f) return flux_of(rR, vnR, t1R, t2R, pR, ER);
+    if (Ss >= 0.0f) return hllc_star(rL, vnL, t1L, t2L, pL, EL, SL, Ss, flux_of(rL, vnL, t1L, t2L, pL, EL));
     return hllc_star(rR, vnR, t1R, t2R, pR, ER, SR, Ss, flux_of(rR, vnR, t1R, t2R, pR, ER));
 }
 
 // HLLC with the face pressures given (the well-balanced z-sweep), hydro_cpu.cpp:75-88.
-template <class R>
-__device__ F5<R> hllc_p(const MatT<R>& m, R rL, R vnL, R t1L, R t2L, R eL, R pL, R rR, R vnR, R t1R, R t2R, R eR,
-                        R pR) {
-    R cL = sound_speed(m, rL, eL), cR = sound_speed(m, rR, eR);
-    if (pL < R(0)) pL = R(0);
-    if (pR < R(0)) pR = R(0);
-    R SL = dmin2(vnL - cL, vnR - cR), SR = dmax2(vnL + cL, vnR + cR);
-    R Ss = (pR - pL + rL * vnL * (SL - vnL) - rR * vnR * (SR - vnR)) / (rL * (SL - vnL) - rR * (SR - vnR));
-    R EL = rL * eL + R(0.5) * rL * (vnL * vnL + t1L * t1L + t2L * t2L),
-      ER = rR * eR + R(0.5) * rR * (vnR * vnR + t1R * t1R + t2R * t2R);
-    if (SL >= R(0)) return flux_of(rL, vnL, t1L, t2L, pL, EL);
-    if (SR <= R(0)) return flux_of(rR, vnR, t1R, t2R, pR, ER);
-    if (Ss >= R(0)) return hllc_star(rL, vnL, t1L, t2L, pL, EL, SL, Ss, flux_of(rL, vnL, t1L, t2L, pL, EL));
+static __device__ F5<float> hllc_p(const MatT<float>& m, float rL, float vnL, float t1L, float t2L, float eL, float pL, float rR, float vnR, float t1R, float t2R, float eR,
+                        float pR) {
+    float cL = sound_speed(m, rL, eL), cR = sound_speed(m, rR, eR);
+    if (pL < 0.0f) pL = 0.0f;
+    if (pR < 0.0f) pR = 0.0f;
+    float SL = dmin2(vnL - cL, vnR - cR), SR = dmax2(vnL + cL, vnR + cR);
+    float Ss = (pR - pL + rL * vnL * (SL - vnL) - rR * vnR * (SR - vnR)) / (rL * (SL - vnL) - rR * (SR - vnR));
+    float EL = rL * eL + 0.5f * rL * (vnL * vnL + t1L * t1L + t2L * t2L),
+      ER = rR * eR + 0.5f * rR * (vnR * vnR + t1R * t1R + t2R * t2R);
+    if (SL >= 0.0f) return flux_of(rL, vnL, t1L, t2L, pL, EL);
+    if (SR <= 0.0f) return flux_of(rR, vnR, t1R, t2R, pR, ER);
+    if (Ss >= 0.0f) return hllc_star(rL, vnL, t1L, t2L, pL, EL, SL, Ss, flux_of(rL, vnL, t1L, t2L, pL, EL));
     return hllc_star(rR, vnR, t1R, t2R, pR, ER, SR, Ss, flux_of(rR, vnR, t1R, t2R, pR, ER));
 }
 
-template <class R>
-__device__ __forceinline__ R mm(R a, R b) {  // minmod, hydro_cpu.cpp:89
-    return (a * b <= R(0)) ? R(0) : (fabs(a) < fabs(b) ? a : b);
+// FP64 fluxes.
+
+// Exact rarefaction into vacuum sampled at the face, hydro_cpu.cpp:43-53.
+static __device__ F5<double> vac_flux(const MatT<double>& m, double rM, double vnM, double t1M, double t2M, double eM, int side) {
+    double pM, cM;
+    eos_pc(m, rM, eM, pM, cM);
+    double g = dv(rM * cM * cM, dmax2(pM, 1e-30));
+    if (lt(g, 1.01)) g = 1.01;
+    if (lt(1e5, g)) g = 1e5;
+    double s = (double)side, vn = s * vnM;
+    if (ge0(vn - cM)) {
+        double E = rM * eM + 0.5 * rM * (vnM * vnM + t1M * t1M + t2M * t2M);
+        return F5<double>{rM * vnM, rM * vnM * vnM + pM, rM * vnM * t1M, rM * vnM * t2M, (E + pM) * vnM};
+    }
+    if (le0(vn + dv(2.0 * cM, g - 1.0))) return F5<double>{0.0, 0.0, 0.0, 0.0, 0.0};
+    double u0 = dv(2.0, g + 1.0) * (cM + 0.5 * (g - 1.0) * vn), c0 = u0;
+    double r0 = rM * pow(dv(c0, cM), dv(2.0, g - 1.0)), p0 = pM * pow(dv(r0, rM), g), e0 = dv(p0, (g - 1.0) * r0),
+      un0 = s * u0;
+    double E0 = r0 * e0 + 0.5 * r0 * (un0 * un0 + t1M * t1M + t2M * t2M);
+    return F5<double>{r0 * un0, r0 * un0 * un0 + p0, r0 * un0 * t1M, r0 * un0 * t2M, (E0 + p0) * un0};
 }
+
+// The HLLC flux of given face states, pressures and sound speeds,
+// hydro_cpu.cpp:54-74 and 75-88.  The flux needs one side only -- which, the
+// wave speeds say -- so the side is chosen first and its terms are formed once
+// (warps with faces of both signs then do not run both).
+static __device__ __forceinline__ F5<double> hllc_pc(double rL, double vnL, double t1L, double t2L, double eL, double pL, double cL, double rR, double vnR, double t1R, double t2R, double eR,
+                                         double pR, double cR) {
+    const double SL = dmin2(vnL - cL, vnR - cR), SR = dmax2(vnL + cL, vnR + cR);
+    const double mL = rL * (SL - vnL), mR = rR * (SR - vnR);  // r (S - vn)
+    const double Ss = dv(pR - pL + rL * vnL * (SL - vnL) - rR * vnR * (SR - vnR), mL - mR);
+    const bool fromL = ge0(SL), fromR = le0(SR);
+    const bool left = fromL || (!fromR && ge0(Ss));
+    const double r = left ? rL : rR, vn = left ? vnL : vnR, t1 = left ? t1L : t1R, t2 = left ? t2L : t2R;
+    const double e = left ? eL : eR, p = left ? pL : pR, S = left ? SL : SR, mS = left ? mL : mR;
+    const double E = r * e + half(r) * (vn * vn + t1 * t1 + t2 * t2);
+    F5<double> F = flux_of(r, vn, t1, t2, p, E);
+    if (fromL || fromR) return F;
+    const double f = dv(mS, S - Ss);
+    const F5<double> Us{f, f * Ss, f * t1, f * t2, f * (dv(E, r) + (Ss - vn) * (Ss + dv(p, mS)))};
+    return F5<double>{F.r + S * (Us.r - r), F.mn + S * (Us.mn - r * vn), F.mt1 + S * (Us.mt1 - r * t1),
+                 F.mt2 + S * (Us.mt2 - r * t2), F.E + S * (Us.E - E)};
+}
+
+// HLLC, hydro_cpu.cpp:54-74.
+static __device__ F5<double> hllc(const MatT<double>& m, double rho_vac, double rL, double vnL, double t1L, double t2L, double eL, double rR, double vnR, double t1R, double t2R,
+                      double eR) {
+    if (rho_vac > 0.0) {
+        bool vL = lt(rL, rho_vac), vR = lt(rR, rho_vac);
+        if (vL && vR) return F5<double>{0.0, 0.0, 0.0, 0.0, 0.0};
+        if (vR) return vac_flux(m, rL, vnL, t1L, t2L, eL, +1);
+        if (vL) return vac_flux(m, rR, vnR, t1R, t2R, eR, -1);
+    }
+    double pL, cL, pR, cR;
+    eos_pc(m, rL, eL, pL, cL);
+    eos_pc(m, rR, eR, pR, cR);
+    return hllc_pc(rL, vnL, t1L, t2L, eL, pL, cL, rR, vnR, t1R, t2R, eR, pR, cR);
+}
+
+// HLLC with the face pressures given (the well-balanced z-sweep), hydro_cpu.cpp:75-88.
+static __device__ F5<double> hllc_p(const MatT<double>& m, double rL, double vnL, double t1L, double t2L, double eL, double pL, double rR, double vnR, double t1R, double t2R, double eR,
+                        double pR) {
+    double q, cL, cR;
+    eos_pc(m, rL, eL, q, cL);
+    eos_pc(m, rR, eR, q, cR);
+    if (lt0(pL)) pL = 0.0;
+    if (lt0(pR)) pR = 0.0;
+    return hllc_pc(rL, vnL, t1L, t2L, eL, pL, cL, rR, vnR, t1R, t2R, eR, pR, cR);
+}
+
+__device__ __forceinline__ float mm(float a, float b) {  // minmod, hydro_cpu.cpp:89
+    return (a * b <= 0.0f) ? 0.0f : (fabsf(a) < fabsf(b) ? a : b);
+}
+__device__ __forceinline__ double mm(double a, double b) { return fi::minmod(a, b); }
 
 // ---------------------------------------------------------------- state
 
@@ -292,6 +496,7 @@ struct Ctl {
     double dt, t, t_end, cfl;
     int64_t steps, max_steps;
     int32_t active, pad;
+    double af_dec;  // exp(-dt / TDEC) of this step (fluidization decay)
     unsigned long long smax_bits;  // CFL speed of this step (positive doubles order as their bits)
     // implicit viscosity: grid barrier of its persistent launch, a wait that
     // ran out (error), conjugate-gradient iterations so far
@@ -306,8 +511,9 @@ static __device__ __forceinline__ int64_t gtid() { return (int64_t)blockIdx.x * 
 
 // hydro_cpu.cpp:94-95
 static __device__ __forceinline__ double eint_of(double r, double mu, double mv, double mw, double E) {
-    double ke = 0.5 * (mu * mu + mv * mv + mw * mw) / r;
-    return (E - ke) / r;
+    const DivBy<double> d = div_by(r);
+    const double ke = dv(half(mu * mu + mv * mv + mw * mw), d);
+    return dv(E - ke, d);
 }
 static __device__ __forceinline__ double pcell(const P& p, const Fields& s, int64_t c) {
     double pr, cs;
@@ -317,34 +523,35 @@ static __device__ __forceinline__ double pcell(const P& p, const Fields& s, int6
 }
 
 // Acoustic fluidization of one cell, hydro_cpu.cpp:390-410.
-static __device__ void update_af_cell(const P& p, const Fields& g, int64_t c, double dt) {
-    const double dec = exp(-dt / p.tdec);
-    double* r = g.q[F_R];
-    double* vib = g.q[F_VIB];
+// dec = exp(-dt / TDEC), the same for every cell.
+static __device__ void update_af_cell(const P& p, const Fields& g, int64_t c, double dec) {
     double* Pmax = g.q[F_PMAX];
-    const double e = eint_of(r[c], g.q[F_MU][c], g.q[F_MV][c], g.q[F_MW][c], g.q[F_E][c]);
+    const double r = g.q[F_R][c], mu = g.q[F_MU][c], mv = g.q[F_MV][c], mw = g.q[F_MW][c];
+    const double pm = Pmax[c];
+    double vib = g.q[F_VIB][c];
+    const double e = eint_of(r, mu, mv, mw, g.q[F_E][c]);
     double Pc, cs;  // Pcell and MAT.sound_speed of the cell
-    eos_pc(p.m, r[c], e, Pc, cs);
-    if (Pc > Pmax[c]) {
-        double dP = Pc - Pmax[c];
+    eos_pc(p.m, r, e, Pc, cs);
+    if (lt(pm, Pc)) {
+        const double dP = Pc - pm;
         Pmax[c] = Pc;
-        if (dP > p.p_act) {
-            double sp = p.af_seeddp ? dP / (dmax2(r[c], 1e-30) * dmax2(cs, 1e-30))
-                                    : sqrt(g.q[F_MU][c] * g.q[F_MU][c] + g.q[F_MV][c] * g.q[F_MV][c] +
-                                           g.q[F_MW][c] * g.q[F_MW][c]) / dmax2(r[c], 1e-30);
-            vib[c] = dmax2(vib[c], p.c_act * sp);
+        if (lt(p.p_act, dP)) {
+            const double sp = p.af_seeddp ? dv(dP, dmax2(r, 1e-30) * dmax2(cs, 1e-30))
+                                          : dv(root(mu * mu + mv * mv + mw * mw), dmax2(r, 1e-30));
+            vib = dmax2(vib, p.c_act * sp);
         }
     }
-    double v0 = vib[c];
-    vib[c] *= dec;
-    double pov = dmax2(Pc, p.p_coh);
+    const double v0 = vib;
+    vib *= dec;
+    const double pov = dmax2(Pc, p.p_coh);
     if (p.af_reg) {
-        if (r[c] > dmax2(p.rho_cfl, 1e-12)) g.q[F_E][c] += 0.5 * r[c] * (v0 * v0 - vib[c] * vib[c]);
-        double vcap = p.af_sat * pov / (dmax2(r[c], 1e-30) * dmax2(cs, 1e-30));
-        if (vib[c] > vcap) vib[c] = vcap;
+        if (r > dmax2(p.rho_cfl, 1e-12)) g.q[F_E][c] += 0.5 * r * (v0 * v0 - vib * vib);
+        const double vcap = dv(p.af_sat * pov, dmax2(r, 1e-30) * dmax2(cs, 1e-30));
+        if (vib > vcap) vib = vcap;
     }
-    double pvib = r[c] * cs * vib[c];
-    g.q[F_AF][c] = pvib / (pvib + pov);
+    g.q[F_VIB][c] = vib;
+    const double pvib = r * cs * vib;
+    g.q[F_AF][c] = dv(pvib, pvib + pov);
 }
 
 // Specific internal energy for an EOS evaluated in R: FP64, the reference's
@@ -356,7 +563,7 @@ static __device__ __forceinline__ double eint_r(double r, double mu, double mv, 
     if constexpr (sizeof(R) == 8) {
         return eint_of(r, mu, mv, mw, E);
     } else {
-        const double inv = 1.0 / r;
+        const double inv = fi::div(1.0, r);
         return (E - 0.5 * (mu * mu + mv * mv + mw * mw) * inv) * inv;
     }
 }
@@ -367,7 +574,7 @@ static __device__ __forceinline__ double pcell_r(const P& p, const Fields& s, in
     const double r = s.q[F_R][c];
     R pr = pressure(mat_of<R>(p), narrow<R>(r),
                     narrow<R>(eint_r<R>(r, s.q[F_MU][c], s.q[F_MV][c], s.q[F_MW][c], s.q[F_E][c])));
-    if (pr < R(0)) pr = R(0);
+    if (lt0(pr)) pr = R(0);
     return widen(pr);
 }
 
@@ -400,7 +607,7 @@ static __device__ void vonmises_cell(const P& p, const Fields& s, const double* 
     if (p.rock) {
         R Pp = R(dmax2(pc.get(p, s, c), 0.0));
         R Peff = Pp;
-        if (p.af_prel && s.q[F_VIB][c] > 0) {
+        if (p.af_prel && gt0(s.q[F_VIB][c])) {
             R p2, cs2;
             eos_pc(mat_of<R>(p), narrow<R>(r),
                    narrow<R>(eint_r<R>(r, s.q[F_MU][c], s.q[F_MV][c], s.q[F_MW][c], s.q[F_E][c])), p2, cs2);
@@ -408,14 +615,15 @@ static __device__ void vonmises_cell(const P& p, const Fields& s, const double* 
         }
         const R mu_i = EU_SETTING(R, mu_i);
         const R ymi = sizeof(R) == 4 ? R(p.cf.ymi) : R(p.y_m - p.y_i0);
-        R Yi = EU_SETTING(R, y_i0) + mu_i * Peff / (R(1) + mu_i * Peff / dmax2(ymi, R(1)));
+        const R mP = mu_i * Peff;
+        R Yi = EU_SETTING(R, y_i0) + dv(mP, R(1) + dv(mP, dmax2(ymi, R(1))));
         R Yd = dmin2(EU_SETTING(R, y_d0) + EU_SETTING(R, mu_d) * Peff, EU_SETTING(R, y_m));
         const R D = narrow<R>(s.q[F_D][c]);
         R Yb = (R(1) - D) * Yi + D * Yd;
         Y = p.af_prel ? Yb : Yb * (R(1) - afc);
-        if (p.y_bingham > 0 && afc > R(1e-3)) {
+        if (p.y_bingham > 0 && lt(R(1e-3), afc)) {
             R Yf = dmin2(EU_SETTING(R, y_bingham), Yb);
-            if (Y < Yf) Y = Yf;
+            if (lt(Y, Yf)) Y = Yf;
         }
     } else {
         Y = (R(1) - narrow<R>(s.q[F_D][c])) * (R(1) - afc) * mat_of<R>(p).Y;
@@ -424,10 +632,10 @@ static __device__ void vonmises_cell(const P& p, const Fields& s, const double* 
                  sxz = s.q[F_SXZ][c], syz = s.q[F_SYZ][c];
     const R xx = narrow<R>(sxx), yy = narrow<R>(syy), zz = narrow<R>(szz), xy = narrow<R>(sxy),
             xz = narrow<R>(sxz), yz = narrow<R>(syz);
-    R J2 = R(0.5) * (xx * xx + yy * yy + zz * zz) + xy * xy + xz * xz + yz * yz;
-    R vm = sqrt(R(3) * J2);
-    if (vm > Y) {
-        const double f = widen(vm > R(0) ? Y / vm : R(0));
+    R J2 = half(xx * xx + yy * yy + zz * zz) + xy * xy + xz * xz + yz * yz;
+    R vm = root(R(3) * J2);
+    if (lt(Y, vm)) {
+        const double f = widen(gt0(vm) ? dv(Y, vm) : R(0));
         s.q[F_SXX][c] = sxx * f; s.q[F_SYY][c] = syy * f; s.q[F_SZZ][c] = szz * f;
         s.q[F_SXY][c] = sxy * f; s.q[F_SXZ][c] = sxz * f; s.q[F_SYZ][c] = syz * f;
         if (p.af_reg && reg && p.m.G > 0 && (p.rho_cfl <= 0 || r > p.rho_cfl)) {
@@ -445,14 +653,14 @@ template <class R>
 static __device__ void grow_damage_cell(const P& p, const Fields& g, int64_t c, double dt, PcellOnce<R>& pc) {
     if (p.m.Emod <= 0 || p.m.wk <= 0) return;
     double* D = g.q[F_D];
-    if (D[c] >= 1.0) return;
+    if (ge(D[c], 1.0)) return;
     const R Pp = R(pc.get(p, g, c));
     const R sigmax = dmax2(-Pp + narrow<R>(g.q[F_SXX][c]),
                            dmax2(-Pp + narrow<R>(g.q[F_SYY][c]), -Pp + narrow<R>(g.q[F_SZZ][c])));
-    if (sigmax > R(0) && sigmax / mat_of<R>(p).Emod > EU_SETTING(R, eps_act)) {
-        R cg = R(0.4) * sqrt(mat_of<R>(p).Emod / dmax2(narrow<R>(g.q[F_R][c]), R(1e-30))),
+    if (gt0(sigmax) && lt(EU_SETTING(R, eps_act), dv(sigmax, mat_of<R>(p).d_Emod))) {
+        R cg = R(0.4) * root(dv(mat_of<R>(p).Emod, dmax2(narrow<R>(g.q[F_R][c]), R(1e-30)))),
           Rs = R(0.5) * EU_SETTING(R, dx);
-        R d13 = pow(narrow<R>(D[c]), R(1) / R(3)) + (cg / Rs) * R(dt);
+        R d13 = pow(narrow<R>(D[c]), R(1) / R(3)) + dv(cg, Rs) * R(dt);
         D[c] = widen(dmin2(R(1), d13 * d13 * d13));
     }
 }
@@ -475,14 +683,15 @@ static __global__ void __launch_bounds__(256) k_maxspeed(P p, Fields g, Ctl* ctl
     double s = 1e-30;
     if (ctl->active && c < p.n) {
         const double r = g.q[F_R][c];
-        if (!(r < p.rho_cfl)) {
+        if (!lt(r, p.rho_cfl)) {
             const double mu = g.q[F_MU][c], mv = g.q[F_MV][c], mw = g.q[F_MW][c];
             const R rr = narrow<R>(r);
             R pr, cs;
             eos_pc(mat_of<R>(p), rr, narrow<R>(eint_r<R>(r, mu, mv, mw, g.q[F_E][c])), pr, cs);
-            R cel = sqrt(cs * cs + (p.m.G > 0 ? R(4.0 / 3.0) * mat_of<R>(p).G / rr : R(0)));
+            const DivBy<R> d = div_by(rr);
+            R cel = root(cs * cs + (p.m.G > 0 ? dv(R(4.0 / 3.0) * mat_of<R>(p).G, d) : R(0)));
             const R fu = narrow<R>(mu), fv = narrow<R>(mv), fw = narrow<R>(mw);
-            R v = sqrt(fu * fu + fv * fv + fw * fw) / rr;
+            R v = dv(root(fu * fu + fv * fv + fw * fw), d);
             s = dmax2(s, widen(v + cel));
         }
     }
@@ -502,6 +711,7 @@ static __global__ void k_dt(P p, Ctl* ctl) {
     double dt = ctl->cfl * p.dx / __longlong_as_double((long long)ctl->smax_bits);
     if (ctl->t + dt > ctl->t_end) dt = ctl->t_end - ctl->t;
     ctl->dt = dt;
+    if (p.tdec > 0) ctl->af_dec = exp(-dt / p.tdec);
 }
 
 static __global__ void k_end(Ctl* ctl) {
@@ -514,7 +724,7 @@ static __global__ void k_end(Ctl* ctl) {
 static __global__ void k_update_af(P p, Fields g, const Ctl* ctl) {
     const int64_t c = gtid();
     if (c >= p.n || !ctl->active) return;
-    update_af_cell(p, g, c, ctl->dt);
+    update_af_cell(p, g, c, ctl->af_dec);
 }
 
 // Primitives of one state (hydro_cpu.cpp:101) and the tracer ratio rc/rho,
@@ -530,7 +740,7 @@ static __global__ void k_prim(P p, Fields s, PrimT<R> W, const Ctl* ctl) {
     const double r = s.q[F_R][c], mu = s.q[F_MU][c], mv = s.q[F_MV][c], mw = s.q[F_MW][c];
     const double E = s.q[F_E][c], rc = s.q[F_RC][c];
     if constexpr (sizeof(R) == 4) {
-        const double inv = 1.0 / r, vx = mu * inv, vy = mv * inv, vz = mw * inv;
+        const double inv = fi::div(1.0, r), vx = mu * inv, vy = mv * inv, vz = mw * inv;
         const double e = (E - 0.5 * (mu * vx + mv * vy + mw * vz)) * inv;
         W.w[0][c] = narrow<R>(r);
         W.w[1][c] = narrow<R>(vx);
@@ -540,26 +750,27 @@ static __global__ void k_prim(P p, Fields s, PrimT<R> W, const Ctl* ctl) {
         W.w[5][c] = narrow<R>(rc * inv);
         if (p.ref_p0) {
             double pr = pressure(p.m, r, e);
-            if (pr < 0) pr = 0;
+            if (lt0(pr)) pr = 0;
             W.w[6][c] = narrow<R>(pr - p.ref_p0[c]);
         }
 #pragma unroll
         for (int q = 0; q < 6; q++) W.sq[q][c] = narrow<R>(s.q[F_SXX + q][c]);
         W.sq[6][c] = narrow<R>(s.q[F_D][c]);
         W.sq[7][c] = narrow<R>(s.q[F_VIB][c]);
-        W.vd[c] = (p.rho_cfl > 0 && r < p.rho_cfl) ? 1 : 0;
+        W.vd[c] = (p.rho_cfl > 0 && lt(r, p.rho_cfl)) ? 1 : 0;
         return;
     }
     W.w[0][c] = R(r);
-    W.w[1][c] = R(mu / r);
-    W.w[2][c] = R(mv / r);
-    W.w[3][c] = R(mw / r);
-    const double e = eint_of(r, mu, mv, mw, E);
+    const DivBy<double> d = div_by(r);  // one divisor for the cell's six quotients
+    W.w[1][c] = R(dv(mu, d));
+    W.w[2][c] = R(dv(mv, d));
+    W.w[3][c] = R(dv(mw, d));
+    const double e = dv(E - dv(half(mu * mu + mv * mv + mw * mw), d), d);
     W.w[4][c] = R(e);
-    W.w[5][c] = R(rc / r);
+    W.w[5][c] = R(dv(rc, d));
     if (p.ref_p0) {  // Pcell - REF_P0 (hydro_cpu.cpp:116)
         double pr = pressure(p.m, r, e);
-        if (pr < 0) pr = 0;
+        if (lt0(pr)) pr = 0;
         W.w[6][c] = R(pr - p.ref_p0[c]);
     }
 }
@@ -616,15 +827,16 @@ static __global__ void __launch_bounds__(256) k_face(P p, PrimT<R> W, FacesT<R> 
     for (int q = 0; q < 5; q++) {
         const R* w = W.w[q];
         const R A = w[cL], B = w[cR], AA = w[cLL], BB = w[cRR];
-        L[q] = A + R(0.5) * mm(A - AA, B - A);
-        Rr[q] = B - R(0.5) * mm(B - A, BB - B);
+        const R mid = B - A;
+        L[q] = add_half(A, mm(A - AA, mid));
+        Rr[q] = sub_half(B, mm(mid, BB - B));
         if (q == 0) {
-            if (L[0] < R(1e-9)) L[0] = A;
-            if (Rr[0] < R(1e-9)) Rr[0] = B;
+            if (lt(L[0], R(1e-9))) L[0] = A;
+            if (lt(Rr[0], R(1e-9))) Rr[0] = B;
         }
         if (q == 4) {
-            if (L[4] < R(0)) L[4] = A;
-            if (Rr[4] < R(0)) Rr[4] = B;
+            if (lt0(L[4])) L[4] = A;
+            if (lt0(Rr[4])) Rr[4] = B;
         }
     }
     constexpr int in = DIR == 0 ? 1 : (DIR == 1 ? 2 : 3), it1 = DIR == 0 ? 2 : 1, it2 = DIR == 2 ? 2 : 3;
@@ -633,9 +845,8 @@ static __global__ void __launch_bounds__(256) k_face(P p, PrimT<R> W, FacesT<R> 
     if (DIR == 2 && p.ref_p0) {  // well-balanced: reconstruct the deviation from the reference (hydro_cpu.cpp:114-119)
         const R* dv = W.w[6];
         const R dLL = dv[cLL], dL = dv[cL], dR = dv[cR], dRR = dv[cRR];
-        const R dLf = dL + R(0.5) * mm(dL - dLL, dR - dL), dRf = dR - R(0.5) * mm(dR - dL, dRR - dR);
-        double p0f = pressure(p.m, 0.5 * (p.ref_r0[cL] + p.ref_r0[cR]), 0.0);
-        if (p0f < 0) p0f = 0;
+        const R dLf = add_half(dL, mm(dL - dLL, dR - dL)), dRf = sub_half(dR, mm(dR - dL, dRR - dR));
+        const double p0f = p.ref_pf[id];
         fl = hllc_p(m, L[0], L[in], L[it1], L[it2], L[4], R(p0f) + dLf, Rr[0], Rr[in], Rr[it1], Rr[it2], Rr[4],
                     R(p0f) + dRf);
     } else {
@@ -646,7 +857,7 @@ static __global__ void __launch_bounds__(256) k_face(P p, PrimT<R> W, FacesT<R> 
     F.q[DIR][2][id] = fl.mt1;
     F.q[DIR][3][id] = fl.mt2;
     F.q[DIR][4][id] = fl.E;
-    F.q[DIR][5][id] = fl.r * (fl.r >= R(0) ? W.w[5][cL] : W.w[5][cR]);
+    F.q[DIR][5][id] = fl.r * (ge0(fl.r) ? W.w[5][cL] : W.w[5][cR]);
 }
 
 // Right-hand side of one cell (hydro_cpu.cpp:98-214): the three directions'
@@ -689,7 +900,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
             const R* const* Fq = F.q[dir];
             R vr, vE, vrc, dmn, dt1, dt2;
             if (dir == 0 && p.axisym) {
-                const R w0 = R(i * p.dx), w1 = R((i + 1) * p.dx), inv = R(1.0 / (((i + 0.5) * p.dx) * p.dx));
+                const R w0 = R(i * p.dx), w1 = R((i + 1) * p.dx), inv = R(fi::div(1.0, ((i + 0.5) * p.dx) * p.dx));
                 vr = -(w1 * Fq[0][b] - w0 * Fq[0][a]) * inv;
                 vE = -(w1 * Fq[4][b] - w0 * Fq[4][a]) * inv;
                 vrc = -(w1 * Fq[5][b] - w0 * Fq[5][a]) * inv;
@@ -698,7 +909,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
                 dt2 = -(w1 * Fq[3][b] - w0 * Fq[3][a]) * inv;
                 R pr, cs;
                 eos_pc(mat_of<R>(p), W.w[0][c], W.w[4][c], pr, cs);  // Pcell: EOS at the cell's internal energy
-                dmn += pr / R((i + 0.5) * p.dx);
+                dmn += dv(pr, R((i + 0.5) * p.dx));
             } else {  // face weights 1 (exact products)
                 const R inv = EU_SETTING(R, invdx);
                 vr = -(Fq[0][b] - Fq[0][a]) * inv;
@@ -734,30 +945,48 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
     // near-void cell (rho < RHO_CFL): the FP32 form reads k_prim's flags
     auto is_void = [&](int64_t q) -> bool {
         if constexpr (sizeof(R) == 4) return W.vd[q] != 0;
-        else return p.rho_cfl > 0 && r[q] < p.rho_cfl;
+        else return p.rho_cfl > 0 && lt(r[q], p.rho_cfl);
+    };
+    // x / dx, and the halved quotient across two cells (x / (2 dx), exactly)
+    auto over_dx = [&](R x) -> R {
+        if constexpr (sizeof(R) == 4) return x / EU_SETTING(R, dx);
+        else return dv(x, p.d_dx);
+    };
+    auto over = [&](R x, bool two) -> R {
+        if constexpr (sizeof(R) == 4) return x / ((two ? R(2) : R(1)) * EU_SETTING(R, dx));
+        else return two ? half(dv(x, p.d_dx)) : dv(x, p.d_dx);
+    };
+    auto third = [&](R x) -> R {
+        if constexpr (sizeof(R) == 4) return x / R(3);
+        else return dv(x, p.d_3);
     };
     if (p.m.G > 0 && !is_void(c)) {  // strength sources, hydro_cpu.cpp:145-213
-        const R G = mat_of<R>(p).G, dx = EU_SETTING(R, dx);
+        const R G = mat_of<R>(p).G;
         const int64_t xm = c - (i > 0 ? plane : 0), xp = c + (i < p.nx - 1 ? plane : 0);
         const int64_t ym = c - (j > 0 ? p.nz : 0), yp = c + (j < p.ny - 1 ? p.nz : 0);
         const int64_t zm = c - (k > 0 ? 1 : 0), zp = c + (k < p.nz - 1 ? 1 : 0);
-        const R hx = ((i > 0 && i < p.nx - 1) ? R(2) : R(1)) * dx, hy = ((j > 0 && j < p.ny - 1) ? R(2) : R(1)) * dx,
-                hz = ((k > 0 && k < p.nz - 1) ? R(2) : R(1)) * dx;
+        const bool hx = i > 0 && i < p.nx - 1, hy = j > 0 && j < p.ny - 1, hz = k > 0 && k < p.nz - 1;
         const R* Vx = W.w[1];  // mu / rho of every cell
         const R* Vy = W.w[2];
         const R* Vz = W.w[3];
         const R vxc = Vx[c], vyc = Vy[c], vzc = Vz[c];
-        auto vxw = [&](int64_t q) { return is_void(q) ? vxc : Vx[q]; };
-        auto vyw = [&](int64_t q) { return is_void(q) ? vyc : Vy[q]; };
-        auto vzw = [&](int64_t q) { return is_void(q) ? vzc : Vz[q]; };
-        const R Lxx = (vxw(xp) - vxw(xm)) / hx, Lxy = (vxw(yp) - vxw(ym)) / hy, Lxz = (vxw(zp) - vxw(zm)) / hz;
-        const R Lyx = (vyw(xp) - vyw(xm)) / hx, Lyy = (vyw(yp) - vyw(ym)) / hy, Lyz = (vyw(zp) - vyw(zm)) / hz;
-        const R Lzx = (vzw(xp) - vzw(xm)) / hx, Lzy = (vzw(yp) - vzw(ym)) / hy, Lzz = (vzw(zp) - vzw(zm)) / hz;
+        const bool oxm = is_void(xm), oxp = is_void(xp), oym = is_void(ym), oyp = is_void(yp), ozm = is_void(zm),
+                   ozp = is_void(zp);
+        auto grad = [&](const R* V, R vc, int64_t q1, bool o1, int64_t q0, bool o0, bool two) {
+            return over((o1 ? vc : V[q1]) - (o0 ? vc : V[q0]), two);
+        };
+        const R Lxx = grad(Vx, vxc, xp, oxp, xm, oxm, hx), Lxy = grad(Vx, vxc, yp, oyp, ym, oym, hy),
+                Lxz = grad(Vx, vxc, zp, ozp, zm, ozm, hz);
+        const R Lyx = grad(Vy, vyc, xp, oxp, xm, oxm, hx), Lyy = grad(Vy, vyc, yp, oyp, ym, oym, hy),
+                Lyz = grad(Vy, vyc, zp, ozp, zm, ozm, hz);
+        const R Lzx = grad(Vz, vzc, xp, oxp, xm, oxm, hx), Lzy = grad(Vz, vzc, yp, oyp, ym, oym, hy),
+                Lzz = grad(Vz, vzc, zp, ozp, zm, ozm, hz);
         const R rcyl = R((i + 0.5) * p.dx);
-        const R eyy = p.axisym ? (vxc / rcyl) : Lyy;
-        const R exx = Lxx, ezz = Lzz, exy = R(0.5) * (Lxy + Lyx), exz = R(0.5) * (Lxz + Lzx),
-                eyz = R(0.5) * (Lyz + Lzy), tr = (exx + eyy + ezz) / R(3);
-        const R Wxy = R(0.5) * (Lxy - Lyx), Wxz = R(0.5) * (Lxz - Lzx), Wyz = R(0.5) * (Lyz - Lzy);
+        const DivBy<R> d_rcyl = div_by(rcyl);
+        const R eyy = p.axisym ? dv(vxc, d_rcyl) : Lyy;
+        const R exx = Lxx, ezz = Lzz, exy = half(Lxy + Lyx), exz = half(Lxz + Lzx), eyz = half(Lyz + Lzy),
+                tr = third(exx + eyy + ezz);
+        const R Wxy = half(Lxy - Lyx), Wxz = half(Lxz - Lzx), Wyz = half(Lyz - Lzy);
         const R* Sxx = W.sq[0];
         const R* Syy = W.sq[1];
         const R* Szz = W.sq[2];
@@ -765,39 +994,47 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
         const R* Sxz = W.sq[4];
         const R* Syz = W.sq[5];
         const R sxx = R(Sxx[c]), syy = R(Syy[c]), szz = R(Szz[c]), sxy = R(Sxy[c]), sxz = R(Sxz[c]), syz = R(Syz[c]);
-        const R Sm[3][3] = {{sxx, sxy, sxz}, {sxy, syy, syz}, {sxz, syz, szz}};
-        const R Wm[3][3] = {{R(0), Wxy, Wxz}, {-Wxy, R(0), Wyz}, {-Wxz, -Wyz, R(0)}};
-        R Jm[3][3];
-#pragma unroll
-        for (int aa = 0; aa < 3; aa++)
-#pragma unroll
-            for (int bb = 0; bb < 3; bb++) {  // (S.W - W.S), hydro_cpu.cpp:172-173
+        R J00, J11, J22, J01, J02, J12;  // S.W - W.S, hydro_cpu.cpp:172-173
+        if constexpr (sizeof(R) == 4) {
+            const R Sm[3][3] = {{sxx, sxy, sxz}, {sxy, syy, syz}, {sxz, syz, szz}};
+            const R Wm[3][3] = {{R(0), Wxy, Wxz}, {-Wxy, R(0), Wyz}, {-Wxz, -Wyz, R(0)}};
+            auto J = [&](int aa, int bb) {
                 R t = R(0);
 #pragma unroll
                 for (int cc = 0; cc < 3; cc++) t += Sm[aa][cc] * Wm[cc][bb] - Wm[aa][cc] * Sm[cc][bb];
-                Jm[aa][bb] = t;
-            }
+                return t;
+            };
+            J00 = J(0, 0); J11 = J(1, 1); J22 = J(2, 2);
+            J01 = J(0, 1); J02 = J(0, 2); J12 = J(1, 2);
+        } else {
+            // without the products with W's zero diagonal; a diagonal entry's
+            // paired products are equal, so each pair is one product doubled
+            const R bxy = sxy * Wxy, bxz = sxz * Wxz, byz = syz * Wyz;
+            J00 = R(-2) * (bxy + bxz); J11 = R(2) * (bxy - byz); J22 = R(2) * (bxz + byz);
+            J01 = sxx * Wxy - Wxy * syy + (-(sxz * Wyz) - Wxz * syz);
+            J02 = sxx * Wxz + (sxy * Wyz - Wxy * syz) - Wxz * szz;
+            J12 = (sxy * Wxz + Wxy * sxz) + syy * Wyz - Wyz * szz;
+        }
         const R u = vxc, v = vyc, w = vzc;
-        const R ix_ = i > 0 ? dx : R(1e30), ixp = i < p.nx - 1 ? dx : R(1e30);
-        const R iy_ = j > 0 ? dx : R(1e30), iyp = j < p.ny - 1 ? dx : R(1e30);
-        const R iz_ = k > 0 ? dx : R(1e30), izp = k < p.nz - 1 ? dx : R(1e30);
+        const bool pu = gt0(u), pv = gt0(v), pw = gt0(w);
+        // the upwind difference's cells; outside the grid the cell itself, so
+        // the difference is zero there
+        const int64_t x1 = pu ? c : xp, x0 = pu ? xm : c, y1 = pv ? c : yp, y0 = pv ? ym : c;
+        const int64_t z1 = pw ? c : zp, z0 = pw ? zm : c;
         auto adv = [&](const R* S) {  // upwind v . grad S, hydro_cpu.cpp:175-178
-            const R sc = R(S[c]);
-            R ax = u > R(0) ? (sc - R(S[xm])) / ix_ : (R(S[xp]) - sc) / ixp;
-            R ay = v > R(0) ? (sc - R(S[ym])) / iy_ : (R(S[yp]) - sc) / iyp;
-            R az = w > R(0) ? (sc - R(S[zm])) / iz_ : (R(S[zp]) - sc) / izp;
-            return u * ax + v * ay + w * az;
+            return u * over_dx(R(S[x1]) - R(S[x0])) + v * over_dx(R(S[y1]) - R(S[y0])) +
+                   w * over_dx(R(S[z1]) - R(S[z0]));
         };
-        dS[0] = A(0) + A(R(2) * G * (exx - tr) + Jm[0][0] - adv(Sxx));
-        dS[1] = A(0) + A(R(2) * G * (eyy - tr) + Jm[1][1] - adv(Syy));
-        dS[2] = A(0) + A(R(2) * G * (ezz - tr) + Jm[2][2] - adv(Szz));
-        dS[3] = A(0) + A(R(2) * G * exy + Jm[0][1] - adv(Sxy));
-        dS[4] = A(0) + A(R(2) * G * exz + Jm[0][2] - adv(Sxz));
-        dS[5] = A(0) + A(R(2) * G * eyz + Jm[1][2] - adv(Syz));
+        dS[0] = A(0) + A(R(2) * G * (exx - tr) + J00 - adv(Sxx));
+        dS[1] = A(0) + A(R(2) * G * (eyy - tr) + J11 - adv(Syy));
+        dS[2] = A(0) + A(R(2) * G * (ezz - tr) + J22 - adv(Szz));
+        dS[3] = A(0) + A(R(2) * G * exy + J01 - adv(Sxy));
+        dS[4] = A(0) + A(R(2) * G * exz + J02 - adv(Sxz));
+        dS[5] = A(0) + A(R(2) * G * eyz + J12 - adv(Syz));
         dD = A(0) + A(-adv(W.sq[6]));
         dvib = A(0) + A(-adv(W.sq[7]));
         // div S into momentum (central differences), hydro_cpu.cpp:183-186
-        auto cd = [&](const R* S, int64_t q1, int64_t q0, R h) { return (R(S[q1]) - R(S[q0])) / h; };
+        auto cd = [&](const R* S, int64_t q1, int64_t q0, bool two) { return over(R(S[q1]) - R(S[q0]), two); };
         const R dSxx_x = cd(Sxx, xp, xm, hx), dSxy_y = cd(Sxy, yp, ym, hy), dSxz_z = cd(Sxz, zp, zm, hz);
         const R dSxy_x = cd(Sxy, xp, xm, hx), dSyy_y = cd(Syy, yp, ym, hy), dSyz_z = cd(Syz, zp, zm, hz);
         const R dSxz_x = cd(Sxz, xp, xm, hx), dSyz_y = cd(Syz, yp, ym, hy), dSzz_z = cd(Szz, zp, zm, hz);
@@ -805,11 +1042,11 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
         dmv += A(dSxy_x + dSyy_y + dSyz_z);
         dmw += A(dSxz_x + dSyz_y + dSzz_z);
         if (p.axisym) {
-            dmu += A((sxx - syy) / rcyl);
-            dmw += A(sxz / rcyl);
+            dmu += A(dv(sxx - syy, d_rcyl));
+            dmw += A(dv(sxz, d_rcyl));
         }
-        if (af[c] > 0 && p.eta_af > 0 && !p.visc_imp) {  // explicit fluidization viscosity, hydro_cpu.cpp:190-197
-            const R eta = R(af[c] * p.eta_af), id2 = R(1.0 / (p.dx * p.dx));
+        if (p.eta_af > 0 && gt0(af[c]) && !p.visc_imp) {  // explicit fluidization viscosity, hydro_cpu.cpp:190-197
+            const R eta = R(af[c] * p.eta_af), id2 = R(p.id2);
             auto vx = [&](int64_t q) { return Vx[q]; };
             auto vy = [&](int64_t q) { return Vy[q]; };
             auto vz = [&](int64_t q) { return Vz[q]; };
@@ -817,16 +1054,16 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
             dmv += A(eta * (vy(xp) + vy(xm) + vy(yp) + vy(ym) + vy(zp) + vy(zm) - R(6) * vy(c)) * id2);
             dmw += A(eta * (vz(xp) + vz(xm) + vz(yp) + vz(ym) + vz(zp) + vz(zm) - R(6) * vz(c)) * id2);
             if (p.axisym) {
-                dmu += A(eta * (Lxx / rcyl - vxc / (rcyl * rcyl)));
-                dmw += A(eta * (Lzx / rcyl));
+                dmu += A(eta * (dv(Lxx, d_rcyl) - dv(vxc, rcyl * rcyl)));
+                dmw += A(eta * dv(Lzx, d_rcyl));
             }
         }
         // div(S.v) into energy, hydro_cpu.cpp:198-203
         auto svx = [&](int64_t q) { return R(Sxx[q]) * Vx[q] + R(Sxy[q]) * Vy[q] + R(Sxz[q]) * Vz[q]; };
         auto svy = [&](int64_t q) { return R(Sxy[q]) * Vx[q] + R(Syy[q]) * Vy[q] + R(Syz[q]) * Vz[q]; };
         auto svz = [&](int64_t q) { return R(Sxz[q]) * Vx[q] + R(Syz[q]) * Vy[q] + R(Szz[q]) * Vz[q]; };
-        dE += A((svx(xp) - svx(xm)) / hx + (svy(yp) - svy(ym)) / hy + (svz(zp) - svz(zm)) / hz);
-        if (p.axisym) dE += A(svx(c) / rcyl);
+        dE += A(over(svx(xp) - svx(xm), hx) + over(svy(yp) - svy(ym), hy) + over(svz(zp) - svz(zm), hz));
+        if (p.axisym) dE += A(dv(svx(c), d_rcyl));
     }
     d.q[D_R][c] = widen(dr);
     d.q[D_MU][c] = widen(dmu);
@@ -844,7 +1081,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? DEU_RHS_MINB_F32 
 // reference (or ambient) density with no energy, stress or tracer,
 // hydro_cpu.cpp:272-290 (not the conservative transfer).
 static __device__ __forceinline__ void void_cell(const P& p, const Fields& g, int64_t c) {
-    if (!(p.rho_cfl > 0 && g.q[F_R][c] < p.rho_cfl)) return;
+    if (!(p.rho_cfl > 0 && lt(g.q[F_R][c], p.rho_cfl))) return;
     if (p.void_cons && p.ref_r0) return;  // the serial conservative pass (k_void_cons) does it
     g.q[F_MU][c] = g.q[F_MV][c] = g.q[F_MW][c] = 0;
     if (p.ref_r0) {
@@ -926,23 +1163,28 @@ static __global__ void k_yield_stage(P p, Fields g1, const double* af, const Ctl
     vonmises_cell<R>(p, g1, af, c, false, pc);
 }
 
-// The reference state's face-pressure difference of the well-balanced gravity
-// source (hydro_cpu.cpp:139-143): p0 at the averaged reference densities of the
-// cell's top and bottom faces (zero internal energy, clamped at 0), in the
-// reference's operation order.  It depends only on the frozen reference and the
-// material, so it is formed once per reference (and material) instead of in
-// every right-hand side.
-static __global__ void k_ref_dp(P p, const double* R0, double* dp) {
+// The reference state's pressure at every z-face (hydro_cpu.cpp:114-119,
+// 139-143): p0 at the averaged reference densities of the two cells, zero
+// internal energy, clamped at 0.  It depends only on the frozen reference and
+// the material, so it is formed once per reference (and material) instead of
+// in every Lop; k_ref_dp differences it over each cell for the well-balanced
+// gravity source.
+static __global__ void k_ref_pf(P p, const double* R0, double* pf) {
+    const int64_t id = gtid();
+    if (id >= (int64_t)p.nx * p.ny * (p.nz + 1)) return;
+    const int64_t line = id / (p.nz + 1);
+    const int f = (int)(id - line * (p.nz + 1));
+    const int64_t base = line * p.nz;
+    const int64_t cL = base + max(0, f - 1), cR = base + min(p.nz - 1, f);
+    double p0 = pressure(p.m, 0.5 * (R0[cL] + R0[cR]), 0.0);
+    if (p0 < 0) p0 = 0;
+    pf[id] = p0;
+}
+static __global__ void k_ref_dp(P p, const double* pf, double* dp) {
     const int64_t c = gtid();
     if (c >= p.n) return;
-    const int k = (int)(c % p.nz);
-    const int64_t ct = c + (k < p.nz - 1 ? 1 : 0), cb = c - (k > 0 ? 1 : 0);
-    double r0t = 0.5 * (R0[c] + R0[ct]), r0b = 0.5 * (R0[cb] + R0[c]);
-    double p0t = pressure(p.m, r0t, 0.0);
-    if (p0t < 0) p0t = 0;
-    double p0b = pressure(p.m, r0b, 0.0);
-    if (p0b < 0) p0b = 0;
-    dp[c] = p0t - p0b;
+    const int64_t f = c + c / p.nz;  // the cell's bottom z-face
+    dp[c] = pf[f + 1] - pf[f];
 }
 
 // set_ref (hydro_cpu.cpp:259-261): density and pressure frozen as the reference.
@@ -982,7 +1224,7 @@ static __global__ void k_correct(P p, Fields g, Fields g1, Rhs d, const Ctl* ctl
 #pragma unroll
         for (int q = 0; q < ND; q++) {
             double* x = g.q[rk_field(q)];
-            x[c] = 0.5 * (x[c] + g1.q[rk_field(q)][c] + dt * d.q[q][c]);
+            x[c] = half(x[c] + g1.q[rk_field(q)][c] + dt * d.q[q][c]);
         }
         if (stage == 1) return;
     }
@@ -1058,8 +1300,9 @@ static __global__ void k_pressure(P p, Fields g, double* out) {
     if (c < p.n) out[c] = pcell(p, g, c);
 }
 
-static __global__ void k_set_step(Ctl* ctl, double dt) {  // a step at a host dt
+static __global__ void k_set_step(P p, Ctl* ctl, double dt) {  // a step at a host dt
     ctl->dt = dt;
+    if (p.tdec > 0) ctl->af_dec = exp(-dt / p.tdec);
     ctl->active = 1;
 }
 static __global__ void k_set_run(Ctl* ctl, double cfl, double t_end, int64_t max_steps) {
