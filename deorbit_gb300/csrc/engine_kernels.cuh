@@ -275,11 +275,27 @@ __device__ __forceinline__ double sep_exact(const View<R>& v, const ImpactD& I, 
     dy = __dsub_rn(v.y[i], v.y[j]);
     dz = __dsub_rn(v.z[i], v.z[j]);
     if constexpr (PER) {
-        if (I.per[0]) { double L = __dsub_rn(I.dhi[0], I.dlo[0]); dx = __dsub_rn(dx, __dmul_rn(L, round(__ddiv_rn(dx, L)))); }
-        if (I.per[1]) { double L = __dsub_rn(I.dhi[1], I.dlo[1]); dy = __dsub_rn(dy, __dmul_rn(L, round(__ddiv_rn(dy, L)))); }
-        if (I.per[2]) { double L = __dsub_rn(I.dhi[2], I.dlo[2]); dz = __dsub_rn(dz, __dmul_rn(L, round(__ddiv_rn(dz, L)))); }
+        if (I.per[0]) { double L = __dsub_rn(I.dhi[0], I.dlo[0]); dx = __dsub_rn(dx, __dmul_rn(L, round(fi::div(dx, L)))); }
+        if (I.per[1]) { double L = __dsub_rn(I.dhi[1], I.dlo[1]); dy = __dsub_rn(dy, __dmul_rn(L, round(fi::div(dy, L)))); }
+        if (I.per[2]) { double L = __dsub_rn(I.dhi[2], I.dlo[2]); dz = __dsub_rn(dz, __dmul_rn(L, round(fi::div(dz, L)))); }
     }
-    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+    return fi::sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+}
+
+// FP64 separation and r^2 of a pair whose neighbour test is settled (by the
+// FP32 distance away from the limit, by sep_exact near it).
+template <bool PER = true, class R>
+__device__ __forceinline__ double sep_sq(const View<R>& v, const ImpactD& I, double xi, double yi, double zi, int64_t j,
+                                         double& dx, double& dy, double& dz) {
+    dx = xi - v.x[j];
+    dy = yi - v.y[j];
+    dz = zi - v.z[j];
+    if constexpr (PER) {
+        if (I.per[0]) { const double L = I.dhi[0] - I.dlo[0]; dx -= L * round(fi::div(dx, L)); }
+        if (I.per[1]) { const double L = I.dhi[1] - I.dlo[1]; dy -= L * round(fi::div(dy, L)); }
+        if (I.per[2]) { const double L = I.dhi[2] - I.dlo[2]; dz -= L * round(fi::div(dz, L)); }
+    }
+    return dx * dx + dy * dy + dz * dz;
 }
 
 // traverse_sphere() on the levels of a graded impact (non-periodic): for every
@@ -1570,13 +1586,16 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
     const float m = sizeof(R) == 8 ? I.margin : 0.0f;
     const R mass_k = v.mass[k];
     const R h0 = I.use_h0 ? v.h0[k] : (R)I.h_init;
+    double xi = 0.0, yi = 0.0, zi = 0.0;
+    if constexpr (sizeof(R) == 8) { xi = v.x[k]; yi = v.y[k]; zi = v.z[k]; }
     R rho = R(1e-30), rho_lo = R(0);
     for (int it = 0; it < iters; it++) {
-        const R ihi = R(1) / hi;
+        const R ihi = rdiv(R(1), hi);
         const bool need_member = 2.0f * (float)hi + 2.0f * m >= I.cwmin * 0.999f;
         AccT<R> sum;
         sum.init();
         const float th2 = (2.0f * (float)hi + m) * (2.0f * (float)hi + m);
+        const float tl = fmaxf(2.0f * (float)hi - m, 0.0f), tl2 = tl * tl;  // surely inside below this
         // mixed form: one entry's m_j W(r, h_i) from its offset record and (mass, cell)
         auto w_mixed = [&](int32_t j, float4 pj, float2 mk) -> float {
             float dx, dy, dz;
@@ -1590,14 +1609,23 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
         };
         auto body = [&](int32_t j) {
             if constexpr (sizeof(R) == 8) {
-                float fx, fy, fz;  // FP32 pre-filter: skip entries that clearly fail
+                // FP32 distance: outside and inside are clear except within the
+                // margin of 2 h, where the reference's exact test decides
+                // (131,072 particles, both iterations: 1.51 -> 0.68 ms with it,
+                // the integer root and the common factors out of the sum)
+                float fx, fy, fz;
                 sep_f32<PER>(I, pi, ci, v.pf[j], v.cpk[j], fx, fy, fz);
-                if (!(fx * fx + fy * fy + fz * fz < th2)) return;
+                const float f2 = fx * fx + fy * fy + fz * fz;
+                if (!(f2 < th2)) return;
                 double dx, dy, dz;
-                double rr = sep_exact<PER>(v, I, k, j, dx, dy, dz);
-                if (!(rr < 2.0 * (double)hi)) return;
+                if (!(f2 < tl2) && !(sep_exact<PER>(v, I, k, j, dx, dy, dz) < 2.0 * (double)hi)) return;
                 if (need_member && !ref_member(bi, v.refbin[j], I)) return;
-                sum.add(v.mass[j] * kernel_W_ih<R>((R)rr, ihi));
+                // 4 pi h^3 W = t^3 - 4 a^3, t = 2 - q, a = max(1 - q, 0)
+                const double q = fi::sqrt(sep_sq<PER>(v, I, xi, yi, zi, j, dx, dy, dz)) * ihi;
+                const double t = 2.0 - q;
+                double a = 1.0 - q;
+                a = fi::lt0(a) ? 0.0 : a;
+                sum.s = fma(v.mass[j], fma(-4.0 * a, a * a, t * t * t), sum.s);
             } else {
                 sum.add((R)w_mixed(j, v.pf[j], v.pk[j]));
             }
@@ -1621,9 +1649,10 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
             traverse<R, LV>(v, I, pi, ci, 2.0f * hf * 1.0001f + 2.0f * I.margin + 1e-6f * hf,
                      [&](int32_t j, float, float, float) { body(j); });
         }
+        if constexpr (sizeof(R) == 8) sum.s *= 0.25 * K<double>::inv_pi * ihi * ihi * ihi;
         rho = rmax(sum.value(), R(1e-30));
         rho_lo = rho > R(1e-30) ? sum.low() : R(0);
-        hi = rmin(R(2) * h0, rmax(R(0.5) * h0, (R)I.eta * rcbrt(mass_k / rho)));
+        hi = rmin(R(2) * h0, rmax(R(0.5) * h0, (R)I.eta * rcbrt(rdiv(mass_k, rho))));
     }
     v.rho[k] = rho;
     v.rho_lo[k] = rho_lo;
@@ -1665,7 +1694,7 @@ static __global__ void k_eos(View<R> v) {
     }
     R P, cs;
     eos_P_cs(m, rho, u, P, cs, rho_lo);
-    const R csig = rsqrt_(cs * cs + (R(4) / R(3)) * m.G / rmax(rho, R(1e-30)));
+    const R csig = rsqrt_(cs * cs + rdiv((R(4) / R(3)) * m.G, rmax(rho, R(1e-30))));
     R pf = P, dsc = R(1);
     R sigmax = R(0);
     if (I.damage_on) {
@@ -1673,9 +1702,9 @@ static __global__ void k_eos(View<R> v) {
         dsc = R(1) - D;
         if (P < R(0)) pf = dsc * P;
     }
-    const R irho2 = R(1) / (rho * rho);
+    const R irho2 = rdiv(R(1), rho * rho);
     const R Rart = (I.eps_as > 0 && pf < R(0)) ? (R)I.eps_as * (-pf) * irho2 : R(0);
-    const R pfr2 = pf * irho2, dsr2 = irho2 * dsc, vol = mass / rho;
+    const R pfr2 = pf * irho2, dsr2 = irho2 * dsc, vol = rdiv(mass, rho);
     v.P[k] = P;
     v.cs[k] = cs;
     v.csig[k] = csig;
@@ -1741,7 +1770,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // entry (cp.async.bulk, TMA), true = six 16-byte cp.async per entry (the load
 // path through L1, completion tracked by cp.async.mbarrier.arrive).
 template <class R, int SE = 0, int SS = 0, bool ASYNC = false, bool LV = false, bool PER = true>
-static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(View<R> v, int32_t* wait_err) {
+static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(View<R> v, int32_t* wait_err) {
     using Acc = AccT<R>;
     constexpr bool kStaged = SS > 0 && sizeof(R) == 4;
     int64_t k = gtid();
@@ -1758,7 +1787,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(Vi
     const R G = v.mats[v.mat[k]].G;
     const bool strength = G > R(0);
     const R alpha = (R)I.alpha, beta = (R)I.beta, eps = (R)I.eps, eps_as = (R)I.eps_as;
-    const R alpha_u = (R)I.alpha_u;
+    const R alpha_u = (R)I.alpha_u, half_alpha = R(0.5) * alpha;
     const R inv_poly = sizeof(R) == 4 ? (R)I.inv_poly_eta_f : (R)I.inv_poly_eta;
     const R hi = v.hh[k], rhoi = v.rho[k], csi = v.csig[k], Pi_over = v.pfr2[k];
     const R dsri = v.dsr2[k], Rai = v.Rart[k];
@@ -1780,49 +1809,15 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(Vi
     const uint32_t ci = v.cpk[k];
     const float m = sizeof(R) == 8 ? I.margin : 0.0f;
     const bool need_member = (float)hi + I.hmax_f + 2.0f * m >= I.cwmin * 0.999f;
-    // one pair's contributions: strain-rate tensor, momentum, energy
-    auto pair_math = [&](R rx, R ry, R rz, R r, R hbar, R ihb, R dW, R gx, R gy, R gz, R vx, R vy, R vz,
-                         R Vj, R rhoj, R csj, R pfj, R dsj, R Raj, R mj, R tjxx, R tjyy, R tjzz, R tjxy,
-                         R tjxz, R tjyz, int32_t j) {
-        if (strength) {
-            const R ex = -vx * Vj, ey = -vy * Vj, ez = -vz * Vj;  // Vj (v_j - v_i)
-            L00 += ex * gx; L01 += ex * gy; L02 += ex * gz;
-            L10 += ey * gx; L11 += ey * gy; L12 += ey * gz;
-            L20 += ez * gx; L21 += ez * gy; L22 += ez * gz;
-        }
-        const R dvr = vx * rx + vy * ry + vz * rz;
-        R Pij = R(0);
-        if (dvr < R(0)) {
-            const R mu = pair_div(hbar * dvr, r * r + eps * hbar * hbar);
-            const R cbar = R(0.5) * (csi + csj);
-            Pij = pair_div(-alpha * cbar * mu + beta * mu * mu, R(0.5) * (rhoi + rhoj));
-        }
-        const R term = Pi_over + pfj + Pij;
-        du.add(R(0.5) * mj * term * (vx * gx + vy * gy + vz * gz));
-        R mterm = term;
-        if (eps_as > R(0)) {
-            const R q = r * ihb;
-            const R t = rmax(R(2) - q, R(0)), a = rmax(R(1) - q, R(0));
-            const R fr = (R(0.25) * t * t * t - a * a * a) * inv_poly;
-            R fn = fr * fr;
-            fn *= fn;
-            mterm += (Rai + Raj) * fn;
-        }
-        const R mm = mj * mterm;
-        const R stx = (sxx * gx + sxy * gy + sxz * gz) * dsri + (tjxx * gx + tjxy * gy + tjxz * gz) * dsj;
-        const R sty = (sxy * gx + syy * gy + syz * gz) * dsri + (tjxy * gx + tjyy * gy + tjyz * gz) * dsj;
-        const R stz = (sxz * gx + syz * gy + szz * gz) * dsri + (tjxz * gx + tjyz * gy + tjzz * gz) * dsj;
-        ax.add(stx * mj - gx * mm);
-        ay.add(sty * mj - gy * mm);
-        az.add(stz * mj - gz * mm);
-        if (alpha_u > R(0)) {
-            const R rbar = R(0.5) * (rhoi + rhoj);
-            // own P and u read here: the conductivity term is off in most runs,
-            // and keeping them live through the pair loop costs registers
-            const R vsig = rsqrt_(pair_div(rabs(v.P[k] - v.P[j]), rbar));
-            du.add(pair_div(alpha_u * mj * vsig * ((R)v.u[k] - (R)v.u[j]) * dW, rbar));
-        }
-    };
+    // FP64 form: own stress over rho^2; the sums carry pi grad W, the energy
+    // sum twice its terms (the common factors are applied once, after the walk)
+    double xi = 0.0, yi = 0.0, zi = 0.0;
+    R oxx = 0, oyy = 0, ozz = 0, oxy = 0, oxz = 0, oyz = 0;
+    if constexpr (sizeof(R) == 8) {
+        xi = v.x[k]; yi = v.y[k]; zi = v.z[k];
+        oxx = sxx * dsri; oyy = syy * dsri; ozz = szz * dsri;
+        oxy = sxy * dsri; oxz = sxz * dsri; oyz = syz * dsri;
+    }
     // mixed form: one list entry's contributions from its six record float4s
     // (global memory or a shared-memory stage); exact zeros for a failing pair
     auto rec_body = [&](int32_t j, const float4 pj, const float4 vhj, const float4 vlj, const float4 fa,
@@ -1893,31 +1888,66 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(Vi
     const float hs_pad = 2.0f * m;
     auto body = [&](int32_t j) {
         if constexpr (sizeof(R) == 8) {
+            // The FP64 pipe bounds the pass (one instruction in 64 cycles on a
+            // sub-partition): divisions, the root and comparisons are integer
+            // work, grad W stays factored as wg d, and the stress and pressure
+            // terms act as one tensor.  131,072 particles with strength: 200 ->
+            // 108 pipe slots a pair, 3.48 -> 1.88 ms (three resident blocks; 2.05
+            // at two, 1.98 at four).
             if (j == (int32_t)k) return;
             const float4 pjf = v.pf[j];
-            float fx, fy, fz;  // FP32 pre-filter: skip entries that clearly fail
+            float fx, fy, fz;  // FP32 distance: the exact test only within its margin of h_i + h_j
             sep_f32<PER>(I, pi, ci, pjf, v.cpk[j], fx, fy, fz);
-            const float lim = pi.w + pjf.w + hs_pad;
-            if (!(fx * fx + fy * fy + fz * fz < lim * lim)) return;
-            const R hj = v.hh[j];
+            const float f2 = fx * fx + fy * fy + fz * fz, lim = pi.w + pjf.w + hs_pad;
+            if (!(f2 < lim * lim)) return;
+            const double hsum = (double)hi + (double)v.hh[j];
             double dx, dy, dz;
-            double rr = sep_exact<PER>(v, I, k, j, dx, dy, dz);
-            double hsum = __dadd_rn((double)hi, (double)hj);
-            if (rr >= hsum || rr == 0.0) return;
+            const float liml = fmaxf(pi.w + pjf.w - hs_pad, 0.0f);
+            if (!(f2 < liml * liml) && fi::le(hsum, sep_exact<PER>(v, I, k, j, dx, dy, dz))) return;
+            const double r2 = sep_sq<PER>(v, I, xi, yi, zi, j, dx, dy, dz);
+            const double r = fi::sqrt(r2);
+            if (fi::bits(r) == 0) return;
             if (need_member && !ref_member(v.refbin[k], v.refbin[j], I)) return;
-            const R rx = (R)dx, ry = (R)dy, rz = (R)dz, r = (R)rr;
-            const R hbar = R(0.5) * (hi + hj);
-            const R ihb = R(1) / hbar;
-            const R dW = kernel_dW_bf<R>(r, ihb);
-            const R wg = dW / r;
-            const R gx = rx * wg, gy = ry * wg, gz = rz * wg;
-            const R vx = (R)(vxi - v.vx[j]), vy = (R)(vyi - v.vy[j]), vz = (R)(vzi - v.vz[j]);
-            const R Vj = v.vol[j], rhoj = v.rho[j], csj = v.csig[j], pfj = v.pfr2[j];
-            const R dsj = v.dsr2[j], Raj = v.Rart[j], mj = v.mass[j];
-            const R tj0 = v.S[0][j], tj1 = v.S[1][j], tj2 = v.S[2][j];
-            const R tj3 = v.S[3][j], tj4 = v.S[4][j], tj5 = v.S[5][j];
-            pair_math(rx, ry, rz, r, hbar, ihb, dW, gx, gy, gz, vx, vy, vz, Vj, rhoj, csj, pfj, dsj, Raj, mj,
-                      tj0, tj1, tj2, tj3, tj4, tj5, j);
+            const double hbar = fi::half(hsum), hb2 = hbar * hbar;
+            const double q = fi::div(r, hbar), t = 2.0 - q;
+            double a = 1.0 - q;
+            a = fi::lt0(a) ? 0.0 : a;
+            const double a2 = a * a, t2 = t * t;
+            const double wg = fi::div(3.0 * a2 - 0.75 * t2, r * (hb2 * hb2));  // pi / r dW/dr
+            const double vx = vxi - v.vx[j], vy = vyi - v.vy[j], vz = vzi - v.vz[j];
+            if (strength) {  // V_j (v_j - v_i) (x) grad W
+                const double vw = -(v.vol[j] * wg);
+                const double ex = vx * vw, ey = vy * vw, ez = vz * vw;
+                L00 += ex * dx; L01 += ex * dy; L02 += ex * dz;
+                L10 += ey * dx; L11 += ey * dy; L12 += ey * dz;
+                L20 += ez * dx; L21 += ez * dy; L22 += ez * dz;
+            }
+            const double dvr = vx * dx + vy * dy + vz * dz;
+            double term = Pi_over + v.pfr2[j];
+            if (fi::lt0(dvr)) {  // artificial viscosity
+                const double mu = fi::div(hbar * dvr, r2 + eps * hb2);
+                term += fi::div(mu * (beta * mu - half_alpha * (csi + v.csig[j])), fi::half(rhoi + v.rho[j]));
+            }
+            const double mj = v.mass[j], mw = mj * wg;
+            du.s += mw * term * dvr;
+            const double Ra = Rai + v.Rart[j];
+            if (fi::bits(Ra) << 1) {  // artificial stress (zero unless one side is in tension)
+                const double fr = (0.25 * t * t2 - a * a2) * inv_poly;
+                const double fr2 = fr * fr;
+                term += Ra * (fr2 * fr2);
+            }
+            const double dsj = v.dsr2[j];
+            const double txy = oxy + v.S[3][j] * dsj, txz = oxz + v.S[4][j] * dsj, tyz = oyz + v.S[5][j] * dsj;
+            const double txx = oxx + v.S[0][j] * dsj - term, tyy = oyy + v.S[1][j] * dsj - term,
+                         tzz = ozz + v.S[2][j] * dsj - term;
+            ax.s += mw * (txx * dx + txy * dy + txz * dz);
+            ay.s += mw * (txy * dx + tyy * dy + tyz * dz);
+            az.s += mw * (txz * dx + tyz * dy + tzz * dz);
+            if (alpha_u > R(0)) {  // conductivity; own P and u read here (off in most runs)
+                const double rbar = fi::half(rhoi + v.rho[j]);
+                const double vsig = fi::sqrt(fi::div(rabs(v.P[k] - v.P[j]), rbar));
+                du.s += fi::div(2.0 * alpha_u * mj * vsig * (v.u[k] - v.u[j]) * (wg * r), rbar);
+            }
         } else {
             // Branch-free: every record of the entry is loaded up front (most
             // entries interact), and a pair that fails the criterion -- or the
@@ -2034,12 +2064,18 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(Vi
         L02 = Lpz.x; L12 = Lpz.y; L22 = Lp22;
         ax.s = kxy.s.x; ay.s = kxy.s.y; az.s = kzu.s.x; du.s = kzu.s.y;
     }
+    if constexpr (sizeof(R) == 8) {
+        const double c = K<double>::inv_pi;
+        L00 *= c; L01 *= c; L02 *= c; L10 *= c; L11 *= c; L12 *= c; L20 *= c; L21 *= c; L22 *= c;
+        ax.s *= c; ay.s *= c; az.s *= c;
+        du.s *= 0.5 * c;
+    }
     R epsw = R(0);
     if (strength) {
         const R exx = L00, eyy = L11, ezz = L22;
         const R exy = R(0.5) * (L01 + L10), exz = R(0.5) * (L02 + L20), eyz = R(0.5) * (L12 + L21);
         const R Rxy = R(0.5) * (L01 - L10), Rxz = R(0.5) * (L02 - L20), Ryz = R(0.5) * (L12 - L21);
-        const R tr = (exx + eyy + ezz) / R(3);
+        const R tr = rdiv(exx + eyy + ezz, R(3));
         // Jaumann J = R S - S R with R = [[0,Rxy,Rxz],[-Rxy,0,Ryz],[-Rxz,-Ryz,0]]
         const R J00 = R(2) * (Rxy * sxy + Rxz * sxz);
         const R J11 = R(2) * (-Rxy * sxy + Ryz * syz);
@@ -2054,7 +2090,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1) k_force(Vi
         v.dS_new[3][k] = twoG * exy + J01;
         v.dS_new[4][k] = twoG * exz + J02;
         v.dS_new[5][k] = twoG * eyz + J12;
-        epsw = (sxx * exx + syy * eyy + szz * ezz + R(2) * (sxy * exy + sxz * exz + syz * eyz)) / rhoi;
+        epsw = rdiv(sxx * exx + syy * eyy + szz * ezz + R(2) * (sxy * exy + sxz * exz + syz * eyz), rhoi);
     } else {
 #pragma unroll
         for (int c = 0; c < 6; c++) v.dS_new[c][k] = R(0);
@@ -2077,9 +2113,9 @@ static __global__ void k_damage(View<R> v) {
     const R D = v.D[k];
     if (m.Emod <= R(0) || D >= R(1)) return;
     const R sig = v.sigmax[k];
-    const R eps_local = sig / m.Emod;
+    const R eps_local = rdiv(sig, m.Emod);
     if (!(sig > R(0) && eps_local > v.eps_act[k])) return;
-    const R cg = R(0.4) * rsqrt_(m.Emod / rmax(v.rho[k], R(1e-30)));
+    const R cg = R(0.4) * rsqrt_(rdiv(m.Emod, rmax(v.rho[k], R(1e-30))));
     const R h0 = I.use_h0 ? v.h0[k] : (R)I.h_init;
     const R Rs = R(0.5) * h0 / (R)I.eta;
     const R dt = (R)I.dt;
@@ -2137,7 +2173,7 @@ static __global__ void k_finish(View<R> v) {
             R J2 = R(0.5) * (s[0] * s[0] + s[1] * s[1] + s[2] * s[2]) + (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
             R vm = rsqrt_(R(3) * J2);
             if (vm > Y) {
-                R f = Y / vm;
+                R f = rdiv(Y, vm);
 #pragma unroll
                 for (int c = 0; c < 6; c++) s[c] *= f;
             }
