@@ -5,17 +5,19 @@
 // Layout: structure of arrays in HBM, one array per field in the reference's
 // cell order (i*ny + j)*nz + k.  One Lop (hydro_cpu.cpp:98-214) is
 //   k_prim   primitives (rho, v, e) and the tracer ratio rc/rho per cell, once
-//            (the reference recomputes them for every face that reads a cell);
-//   k_face   one launch per direction, one thread per face: MUSCL-minmod
-//            reconstruction from four cells, HLLC (or the vacuum flux), the
-//            tracer flux -- each face flux computed once and stored;
-//   k_rhs    one thread per cell: the three directions' flux differences added
-//            in the reference's order (x, y, z), gravity, then the strength
-//            sources (Jaumann rate, upwind advection, div S, div(S.v)).
+//            (the reference recomputes them for every face that reads a cell),
+//            after the cell's fluidization update; the predictor's primitives
+//            are formed by k_predict itself;
+//   k_face   one thread per face: MUSCL-minmod reconstruction from four cells,
+//            HLLC (or the vacuum flux), the tracer flux -- each face flux
+//            computed once and stored; no sweep along an axis of one cell;
+//   k_rhs    one thread per cell and part: the directions' flux differences
+//            added in the reference's order (x, y, z), gravity, then the
+//            strength sources (Jaumann rate, upwind advection, div S, div(S.v)).
 // The Runge-Kutta stages (k_predict, k_correct) fuse the elementwise updates
 // with the void-cell reset, the radial return, damage growth and damping.
-// k_maxspeed reduces the CFL speed; k_dt forms dt and the stop test on the
-// device, so whole steps replay from a captured CUDA graph.
+// k_maxspeed reduces the CFL speed and forms dt; k_end advances the time and
+// holds the stop test, so whole steps replay from a captured CUDA graph.
 //
 // This file is compiled without fused multiply-adds (--fmad=false): every
 // expression is evaluated in the reference's operation order with IEEE
@@ -415,12 +417,13 @@ struct Grid {
     cudaStream_t st = nullptr;
     P p{};
     Fields g{}, g1{};
-    Rhs d{};
+    RhsT<double> d{};          // right-hand side, FP64 form
     bool mixed = false;        // Lop in FP32 (primitives, face fluxes, sources)
     PrimT<double> W{};         // FP64 form
     FacesT<double> F{};
     PrimT<float> W32{};        // mixed form
     FacesT<float> F32{};
+    RhsT<float> d32{};
     Ctl* ctl = nullptr;
     double* scratch = nullptr;  // pressure read-out
     double* ref_r0 = nullptr;   // hydrostatic reference (set_ref), allocated on first use
@@ -435,8 +438,6 @@ struct Grid {
     bool graph_valid = false;
     int64_t graph_launches = 0;  // kernels per replay of the step graph
     Visc vw{};                   // implicit viscosity work arrays, allocated on first use
-    FaceFork fork{};             // side streams for the face passes (small grids)
-    bool fork_faces = false;
     int pin_floor = 0;           // driver adjustments after each step (eu_set_driver)
     int sponge_from = -1;
     int driver_flags = 0;
@@ -457,10 +458,6 @@ struct Grid {
         if (graph) cudaGraphExecDestroy(graph);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {fork.fork, fork.join[0], fork.join[1]})
-            if (e) cudaEventDestroy(e);
-        for (cudaStream_t s2 : fork.side)
-            if (s2) cudaStreamDestroy(s2);
         for (void* a : allocs) cudaFree(a);
         allocs.clear();
         if (st) cudaStreamDestroy(st);
@@ -503,38 +500,36 @@ struct Grid {
         launches++;
     }
 
+    // Primitives of the state s (with its update_af first), then the Lop of s.
+    void enqueue_prim(const Fields& s, int af) {
+        if (mixed) enqueue_prim_f32(p, s, W32, ctl, st, af);
+        else enqueue_prim_t<double>(p, s, W, ctl, st, af);
+        launches++;
+    }
     void enqueue_lop(const Fields& s) {
-        const FaceFork* fk = fork_faces ? &fork : nullptr;
-        EU_CUDA(mixed ? enqueue_lop_f32(p, s, W32, g.q[F_AF], F32, d, ctl, st, fk)
-                      : enqueue_lop_t<double>(p, s, W, g.q[F_AF], F, d, ctl, st, fk));
-        launches += 5;
+        launches += mixed ? enqueue_lop_f32(p, s, W32, g.q[F_AF], F32, d32, ctl, st)
+                          : enqueue_lop_t<double>(p, s, W, g.q[F_AF], F, d, ctl, st);
     }
 
     // One step_rk2 (hydro_cpu.cpp:411-425); with_dt: the drivers' dt and stop
     // test on the device first.
     void enqueue_step(bool with_dt) {
-        const int64_t n = p.n;
         if (with_dt) {
-            k_begin<<<1, 1, 0, st>>>(ctl);
-            if (mixed) enqueue_maxspeed_f32(p, g, ctl, st);
-            else enqueue_maxspeed_t<double>(p, g, ctl, st);
-            k_dt<<<1, 1, 0, st>>>(p, ctl);
-            launches += 3;
-        }
-        if (p.c_act > 0 && p.tdec > 0) {
-            k_update_af<<<grid_of(n), 256, 0, st>>>(p, g, ctl);
+            if (mixed) enqueue_maxspeed_f32(p, g, ctl, st, 1);
+            else enqueue_maxspeed_t<double>(p, g, ctl, st, 1);
             launches++;
         }
+        enqueue_prim(g, p.c_act > 0 && p.tdec > 0);
         enqueue_lop(g);
-        if (mixed) enqueue_predict_f32(p, g, g1, d, ctl, st);
-        else enqueue_predict_t<double>(p, g, g1, d, ctl, st);
+        if (mixed) enqueue_predict_f32(p, g, g1, W32, d32, ctl, st);
+        else enqueue_predict_t<double>(p, g, g1, W, d, ctl, st);
         enqueue_lop(g1);
         const bool vi = visc_on();
-        if (mixed) enqueue_correct_f32(p, g, g1, d, ctl, st, vi ? 1 : 0);
+        if (mixed) enqueue_correct_f32(p, g, g1, d32, ctl, st, vi ? 1 : 0);
         else enqueue_correct_t<double>(p, g, g1, d, ctl, st, vi ? 1 : 0);
         if (vi) {  // implicit_visc between the average and the rest (hydro_cpu.cpp:420)
             enqueue_visc();
-            if (mixed) enqueue_correct_f32(p, g, g1, d, ctl, st, 2);
+            if (mixed) enqueue_correct_f32(p, g, g1, d32, ctl, st, 2);
             else enqueue_correct_t<double>(p, g, g1, d, ctl, st, 2);
             launches++;
         }
@@ -643,6 +638,7 @@ void derive(deu::P& p) {
     p.d_dx = deu::div_by(p.dx);
     p.d_3 = deu::div_by(3.0);
     p.id2 = 1.0 / (p.dx * p.dx);
+    p.flat = (p.nx == 1 && !p.axisym ? 1 : 0) | (p.ny == 1 ? 2 : 0) | (p.nz == 1 ? 4 : 0);
     p.eps_act = (m.Emod > 0 && m.wk > 0) ? std::pow(1.0 / (m.wk * p.dx * p.dx * p.dx), 1.0 / m.wm) : 0.0;
     p.invdx = 1.0 / p.dx;
     p.cf.y_i0 = (float)p.y_i0; p.cf.mu_i = (float)p.mu_i; p.cf.ymi = (float)(p.y_m - p.y_i0);
@@ -681,6 +677,11 @@ int eu_create_form(int32_t nx, int32_t ny, int32_t nz, double dx, int32_t device
         if (!(dx > 0) || !std::isfinite(dx)) throw SphError(SPH_ERR_ARG, "dx must be finite and > 0");
         const int64_t n = (int64_t)nx * ny * nz;
         if (n > ((int64_t)1 << 31) - 1) throw SphError(SPH_ERR_CAPACITY, "more than 2^31 - 1 cells");
+        // FP32 columns are addressed with 32-bit byte offsets (some 100 columns of
+        // this size would exceed every device's memory by far)
+        const int64_t most_faces = n + std::max({(int64_t)ny * nz, (int64_t)nx * nz, (int64_t)nx * ny});
+        if (form == EU_MIXED && most_faces >= (int64_t)1 << 30)
+            throw SphError(SPH_ERR_NOMEM, "device allocation failed: grid larger than the device's memory");
         int ndev = 0;
         cudaError_t e = cudaGetDeviceCount(&ndev);
         if (e != cudaSuccess || ndev == 0)
@@ -701,8 +702,11 @@ int eu_create_form(int32_t nx, int32_t ny, int32_t nz, double dx, int32_t device
             for (int q = 0; q < deu::NF; q++) g->g.q[q] = g->alloc(n);
             for (int q = 0; q < deu::NF; q++) g->g1.q[q] = g->g.q[q];  // af, Pmax shared
             for (int q = 0; q < deu::ND; q++) g->g1.q[deu::rk_field(q)] = g->alloc(n);
-            for (int q = 0; q < deu::ND; q++) g->d.q[q] = g->alloc(n);
             g->mixed = form == EU_MIXED;
+            for (int q = 0; q < deu::ND; q++) {
+                if (g->mixed) g->d32.q[q] = g->alloc<float>(n);
+                else g->d.q[q] = g->alloc(n);
+            }
             for (int q = 0; q < 7; q++) {
                 if (g->mixed) g->W32.w[q] = g->alloc<float>(n);
                 else g->W.w[q] = g->alloc(n);
@@ -726,16 +730,6 @@ int eu_create_form(int32_t nx, int32_t ny, int32_t nz, double dx, int32_t device
             g->ctl = (deu::Ctl*)c;
             EU_CUDA(cudaMemsetAsync(c, 0, sizeof(deu::Ctl), g->st));
             for (auto& ev : g->ev) EU_CUDA(cudaEventCreate(&ev));
-            // Small grids: the three face passes of a Lop fill the device only
-            // side by side (a pass of a 2-D grid is a few dozen blocks).
-            int nsm = 0;
-            EU_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-            g->fork_faces = n < (int64_t)nsm * 256 * 8;
-            if (g->fork_faces) {
-                for (auto& s2 : g->fork.side) EU_CUDA(cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking));
-                EU_CUDA(cudaEventCreateWithFlags(&g->fork.fork, cudaEventDisableTiming));
-                for (auto& e : g->fork.join) EU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            }
             EU_CUDA(cudaStreamSynchronize(g->st));
         } catch (...) {
             g->release();
@@ -892,6 +886,7 @@ int eu_lop(eu_grid* h) {
         deu::Grid* g = G(h);
         deu::DeviceScope ds(g->device);
         deu::k_maxspeed_begin<<<1, 1, 0, g->st>>>(g->ctl);  // marks the control active
+        g->enqueue_prim(g->g, 0);
         g->enqueue_lop(g->g);
         g->launches++;
         g->check();
@@ -906,7 +901,14 @@ int eu_read_rhs(eu_grid* h, const char* name, double* host, int64_t n) {
         if (!host) throw SphError(SPH_ERR_ARG, "null host buffer");
         deu::DeviceScope ds(g->device);
         const int q = deu::rhs_index(name);
-        EU_CUDA(cudaMemcpyAsync(host, g->d.q[q], sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, g->st));
+        const double* src = g->d.q[q];
+        if (g->mixed) {
+            deu::k_widen<<<g->grid_of(n), 256, 0, g->st>>>(g->d32.q[q], g->scratch, n);
+            g->launches++;
+            g->check();
+            src = g->scratch;
+        }
+        EU_CUDA(cudaMemcpyAsync(host, src, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, g->st));
         EU_CUDA(cudaStreamSynchronize(g->st));
     });
 }
@@ -955,8 +957,8 @@ int eu_maxspeed(eu_grid* h, double* out) {
         if (!out) throw SphError(SPH_ERR_ARG, "null output pointer");
         deu::DeviceScope ds(g->device);
         deu::k_maxspeed_begin<<<1, 1, 0, g->st>>>(g->ctl);
-        if (g->mixed) deu::enqueue_maxspeed_f32(g->p, g->g, g->ctl, g->st);
-        else deu::enqueue_maxspeed_t<double>(g->p, g->g, g->ctl, g->st);
+        if (g->mixed) deu::enqueue_maxspeed_f32(g->p, g->g, g->ctl, g->st, 0);
+        else deu::enqueue_maxspeed_t<double>(g->p, g->g, g->ctl, g->st, 0);
         g->launches += 2;
         g->check();
         const deu::Ctl c = g->read_ctl();

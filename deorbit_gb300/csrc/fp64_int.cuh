@@ -33,7 +33,11 @@ namespace fi {
 
 FI_FN uint64_t bits(double x) {
 #ifdef __CUDA_ARCH__
-    return (uint64_t)__double_as_longlong(x);
+    // opaque to the compiler, which turns integer tests of a double's bits
+    // (zero, NaN) back into comparisons on the FP64 pipe
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+    return (uint64_t)hi << 32 | lo;
 #else
     uint64_t b;
     std::memcpy(&b, &x, 8);
@@ -127,24 +131,27 @@ FI_FN Divisor divisor(double b) {
     return d;
 }
 
+// The hardware's operations for what the integer ones leave out.  Calls, not
+// inline code: the compiler would otherwise issue the FP64 instruction in every
+// case and select.
 #ifdef __CUDACC__
-static __device__ __noinline__ double div_hw(double a, double b) { return __ddiv_rn(a, b); }
-static __device__ __noinline__ double sqrt_hw(double a) { return __dsqrt_rn(a); }
-#endif
-FI_FN double div_general(double a, double b) {
-#ifdef __CUDA_ARCH__
-    return div_hw(a, b);
+#define FI_RARE static __host__ __device__ __noinline__
 #else
-    return a / b;
+#define FI_RARE static
 #endif
-}
-FI_FN double sqrt_general(double a) {
+FI_RARE double div_general(double a, double b) { return a / b; }
+FI_RARE double sqrt_general(double a) {
 #ifdef __CUDA_ARCH__
-    return sqrt_hw(a);
+    return __dsqrt_rn(a);
 #else
     return std::sqrt(a);
 #endif
 }
+FI_RARE double half_general(double x) { return 0.5 * x; }
+FI_RARE float to_float_general(double x) { return (float)x; }
+FI_RARE double to_double_general(float y) { return (double)y; }
+FI_RARE bool product_le0(double a, double b) { return a * b <= 0; }
+
 // a / d, rounded to nearest even (a tie cannot occur: it would need a divisor
 // significand with a factor 2^53).
 FI_FN double div(double a, const Divisor& d) {
@@ -226,7 +233,28 @@ FI_FN bool abs_lt(double a, double b) { return (bits(a) << 1) < (bits(b) << 1) &
 FI_FN double half(double x) {
     const uint32_t e = (hi32(bits(x)) >> 20) & 0x7ffu;
     if (e - 2u < 0x7fdu) return from_bits(bits(x) - 0x10000000000000ull);
-    return (bits(x) << 1) == 0 || e == 0x7ffu ? x : 0.5 * x;
+    return (bits(x) << 1) == 0 || e == 0x7ffu ? x : half_general(x);
+}
+
+// Conversions (FP64-pipe instructions in hardware): to nearest even, and exact.
+// Results or operands below FP32's normal range, infinities and NaN take the
+// hardware's.
+FI_FN float to_float(double x) {
+    const uint64_t u = bits(x);
+    const uint32_t e = (hi32(u) >> 20) & 0x7ffu, rest = lo32(u) << 3;
+    uint32_t f = (uint32_t)((u & 0x7fffffffffffffffull) >> 29) - (896u << 23);
+    f += rest + (f & 1u) > 0x80000000u ? 1u : 0u;
+    const bool zero = (u << 1) == 0;
+    if (zero) f = 0;
+    if (!zero && !(e - 897u < 254u)) return to_float_general(x);
+    return bits_f(f | (hi32(u) & 0x80000000u));
+}
+FI_FN double to_double(float y) {
+    const uint32_t f = f_bits(y), a = f & 0x7fffffffu;
+    const bool zero = a == 0;
+    if (!zero && !(a - 0x800000u < 0x7f000000u)) return to_double_general(y);
+    const uint32_t h = zero ? 0u : (a >> 3) + (896u << 20);
+    return from_bits(((uint64_t)(h | (f & 0x80000000u)) << 32) | (uint64_t)(f << 29));
 }
 
 // minmod: 0 where a b <= 0, else the smaller of the two in magnitude (b where
@@ -236,7 +264,7 @@ FI_FN double minmod(double a, double b) {
     const uint32_t ea = (hi32(bits(a)) >> 20) & 0x7ffu, eb = (hi32(bits(b)) >> 20) & 0x7ffu;
     const bool zero = (bits(a) << 1) == 0 || (bits(b) << 1) == 0;
     if (ea == 0x7ffu || eb == 0x7ffu || (!zero && ea + eb < 1023u)) {
-        if (a * b <= 0) return 0.0;
+        if (product_le0(a, b)) return 0.0;
     } else if (zero || ((hi32(bits(a)) ^ hi32(bits(b))) >> 31)) {
         return 0.0;
     }

@@ -36,6 +36,9 @@ int main(int, char** v) {
         if (mode == 6) a = (((b & frac) + g() % 5 - 2) & frac) | (1023ull << 52);
         if (mode == 7 && (i & 8)) a &= 1ull << 63;
         double x = fi::from_bits(a), y = fi::from_bits(b);
+        if (mode == 2) a = (a & 0x800fffffffffffffull) | ((1023 - 152 + g() % 285) << 52);  // FP32's range and edges
+        if (mode == 2 && (i & 16)) a = (a & ~0x3fffffffull) | 0x10000000ull;  // ties of the conversion
+        if (mode == 2) x = fi::from_bits(a);
         if (mode == 8) { x = sp[g() % 15]; if (g() & 1) y = sp[g() % 15]; if (g() % 7 == 0) x = y; }
         const double mm = (x * y <= 0) ? 0.0 : (std::fabs(x) < std::fabs(y) ? x : y);
         const double m = fi::minmod(x, y);
@@ -43,7 +46,8 @@ int main(int, char** v) {
                          fi::gt0(x) == (x > 0) && fi::ge0(x) == (x >= 0) && fi::le0(x) == (x <= 0) &&
                          fi::abs_lt(x, y) == (std::fabs(x) < std::fabs(y));
         if (!same(fi::div(x, y), x / y) || !cmp || !(same(m, mm) || (m == 0 && mm == 0)) ||
-            !same(fi::half(x), 0.5 * x)) {
+            !same(fi::half(x), 0.5 * x) || !same(fi::to_float(x), (float)x) ||
+            !same(fi::to_double((float)y), (double)(float)y)) {
             std::printf("%a %a\n", x, y);
             return 1;
         }
