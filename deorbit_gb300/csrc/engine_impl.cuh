@@ -256,15 +256,6 @@ static __global__ void __launch_bounds__(512) k_diagnostics(View<R> v, int b, in
     }
 }
 
-// After a sort: offsets change, and positions may have (bins are stale).
-static __global__ void k_impact_reset_omax(ImpactD* imps, int nimp) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < nimp) {
-        imps[b].omax_bits = 0u;
-        imps[b].bins_ok = 0;
-    }
-}
-
 static __global__ void k_set_mask_dt(ImpactD* imps, int nimp, const int32_t* mask, const double* dt,
                               const double* t_end) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -570,9 +561,9 @@ public:
     int64_t bytes_per_particle() const {
         const int64_t R4 = sizeof(R) == 4;
         int64_t b = 2 * (kND * 8 + kNR * (int64_t)sizeof(R) + 1 + 1 + 2 + 4) + kNDer * (int64_t)sizeof(R);
-        b += 16 + 16 + 4 + 8 * R4 + 16 + 96 * R4 + 4 + 4 + 8 + 4 + 4 + 4 + 4 + 4 * kExtraCap;
+        b += 16 + 16 + 4 + 8 * R4 + 16 + 96 * R4 + 4 + 4 + 8 + 16 + 4 + 4 + 4 + 4 * kExtraCap;
         b += 16 * (((int64_t)cap_nbr_ + 3) / 4);
-        b += 4 + 12 + 8;  // pos_of_gid, three key arrays, two id arrays
+        b += 4;  // pos_of_gid
         return b;
     }
     int64_t device_bytes() override { return dev_bytes_; }
@@ -681,8 +672,8 @@ public:
             }
         if (!any) return;
         set_masks(mask, nullptr, nullptr);
-        sort_reorder(true);
-        build_list<kListSuperset>(true);
+        sort_reorder(true, true);
+        build_list<kListSuperset>(true, true);
         density_rounds(2, true);
         forces(true);
         launch_n(k_adopt_derivatives<R>, N_);
@@ -732,39 +723,40 @@ public:
     // before_eos (optional) runs between the head (kick, drift, sort, list,
     // density rounds: x, y, z and h final, u, D and S not yet read) and the
     // tail (EOS, forces, damage, finish, dt).
-    void one_step(bool host_sync, const std::function<void()>* before_eos = nullptr) {
+    // between: another step of the same graph follows.
+    void one_step(bool host_sync, const std::function<void()>* before_eos = nullptr, bool between = false) {
         step_head(host_sync);
         if (before_eos) (*before_eos)();
-        step_tail();
+        step_tail(!host_sync, between);
     }
     void step_head(bool host_sync) {
         if (profiling_) DSPH_CUDA(cudaEventRecord(ev_[0], st_));
         cls(KC_KICK);
-        launch_n(k_kick_drift<R>, N_);
-        sort_reorder(false);
+        launch_kick();
+        sort_reorder(false, true, true);
         cls(KC_LIST_DENSITY);
-        build_list<kListSuperset>(false);
+        build_list<kListSuperset>(false, true);
         if (profiling_) DSPH_CUDA(cudaEventRecord(ev_[1], st_));
         density_rounds(2, host_sync);
         if (profiling_) DSPH_CUDA(cudaEventRecord(ev_[2], st_));
         if (host_sync) refresh_list_if_needed();
         else refresh_list_device();
     }
-    void step_tail() {
+    // refreshed: the head rebuilt the lists that its density rounds outgrew on
+    // the device (captured heads).
+    void step_tail(bool refreshed, bool between = false) {
+        refreshed = refreshed && list_mode_ == 0;
         const int nimp = (int)imp_.size();
         cls(KC_EOS);
-        launch_n(k_eos<R>, N_);
+        launch_eos(refreshed);
         if (profiling_) DSPH_CUDA(cudaEventRecord(ev_[3], st_));
         cls(KC_FORCE);
         launch_force();
         if (profiling_) DSPH_CUDA(cudaEventRecord(ev_[4], st_));
-        cls(KC_DAMAGE);
-        launch_n(k_damage<R>, N_);
         cls(KC_FINISH);
         launch_n(k_finish<R>, N_);
         cls(KC_DT);
-        dt_reduce();
-        launch_small(k_run_control, nimp, 1);
+        launch_small(k_run_control, nimp, between ? 2 : 1);
         cls(KC_OTHER);
         if (profiling_) {
             DSPH_CUDA(cudaEventRecord(ev_[5], st_));
@@ -865,11 +857,11 @@ public:
                 break;
             }
             if (kind == kGraphTail) {
-                step_tail();
+                step_tail(true);
                 break;
             }
-            if (kind != kGraphHostDt) launch_small(k_run_control, nimp, 0);
-            one_step(false);
+            if (kind != kGraphHostDt && k == 0) launch_small(k_run_control, nimp, 0);
+            one_step(false, nullptr, kind == kGraphTwo && k == 0);
         }
         cudaGraph_t g = nullptr;
         DSPH_CUDA(cudaStreamEndCapture(st_, &g));
@@ -902,8 +894,8 @@ public:
     void compute_density_h(int iters) override {
         commit();
         set_all_masks();
-        sort_reorder(true);
-        build_list<kListSuperset>(true);
+        sort_reorder(true, true);
+        build_list<kListSuperset>(true, true);
         density_rounds(iters, true);
         check_async();
     }
@@ -913,7 +905,7 @@ public:
         set_all_masks();
         if (!grid_valid_) {
             sort_reorder(true);
-            build_list<kListSuperset>(true);
+            build_list<kListSuperset>(true, true);
             final_grid_build();
         }
         forces(true);
@@ -1975,8 +1967,7 @@ public:
     }
 
     void ensure_scratch() {
-        size_t need = std::max(radix_scratch_bytes(std::max<int64_t>(Gcap_, 1)),
-                               scan_scratch_bytes(std::max<int64_t>(Ccap_, 1))) + 256;
+        size_t need = scan_scratch_bytes(std::max<int64_t>(Ccap_, 1)) + 256;
         if (need > scratch_bytes_) {
             dfree(scratch_);
             scratch_bytes_ = need;
@@ -2027,8 +2018,6 @@ public:
         DSPH_CUDA(cudaStreamSynchronize(st_));
         dfree(pos_of_gid_);
         pos_of_gid_ = npos;
-        for (uint32_t** p : {&keys_by_gid_, &skeys_, &tkeys_}) { dfree(*p); *p = dalloc<uint32_t>(nc); }
-        for (int32_t** p : {&sgid_, &tgid_}) { dfree(*p); *p = dalloc<int32_t>(nc); }
         Gcap_ = nc;
         ensure_scratch();
     }
@@ -2065,7 +2054,8 @@ public:
         dfree(tasks_); tasks_ = dalloc<int32_t>(nc);
         dfree(cpk_); cpk_ = dalloc<uint32_t>(nc);
         dfree(refbin_); refbin_ = dalloc<unsigned long long>(nc);
-        dfree(src_); src_ = dalloc<int32_t>(nc);
+        dfree(key_rank_); key_rank_ = dalloc<uint2>(nc);
+        dfree(slot_); slot_ = dalloc<int2>(nc);
         dfree(nbr_cnt_); nbr_cnt_ = dalloc<int32_t>(nc);
         dfree(hlist_); hlist_ = dalloc<float>(nc);
         dfree(xcnt_); xcnt_ = dalloc<int32_t>(nc);
@@ -2324,14 +2314,34 @@ public:
         set_masks(mask, nullptr, nullptr);
     }
 
-    int key_bits() const {
-        int bits = 1;
-        while ((1ll << bits) <= C_) bits++;
-        return bits;
+    unsigned blocks_of(int64_t n) const { return (unsigned)((n + 255) / 256); }
+
+    void launch_kick() {
+        if (N_ <= 0) return;
+        const int nimp = (int)imp_.size();
+        const unsigned nb = blocks_of(N_);
+        prof_begin();
+        k_kick_drift<R><<<nb + blocks_of(nimp), 256, 0, st_>>>(view(), nb, nimp);
+        launched((const void*)k_kick_drift<R>);
+        prof_end();
+        launches_++;
+    }
+
+    void launch_eos(bool refreshed) {
+        if (N_ <= 0) return;
+        const int nimp = (int)imp_.size();
+        const unsigned nb = blocks_of(N_);
+        prof_begin();
+        k_eos<R><<<nb + blocks_of(nimp), 256, 0, st_>>>(view(), nb, nimp, refreshed ? 1 : 0);
+        launched((const void*)k_eos<R>);
+        prof_end();
+        launches_++;
     }
 
     // Cell sort of all resident particles and gather of the carried state.
-    void sort_reorder(bool count_changes) {
+    // rounds: density rounds follow (the first round's reference grid and bins
+    // are made on the way); begun: the kick did sort_begin.
+    void sort_reorder(bool count_changes, bool rounds = false, bool begun = false) {
         if (N_ == 0 && !count_changes) return;
         if (G_ == 0) {  // no particle was ever added: nothing to order
             N_ = 0;
@@ -2339,15 +2349,12 @@ public:
             return;
         }
         const int nimp = (int)imp_.size();
-        DSPH_CUDA(cudaMemsetAsync(keys_by_gid_, 0xff, sizeof(uint32_t) * std::max<int64_t>(G_, 1), st_));
         DSPH_CUDA(cudaMemsetAsync(cell_cnt_, 0, sizeof(int32_t) * (C_ + 1), st_));
         const int keep_cls = cur_cls_;
         cls(KC_SORT);
-        launch_small(k_impact_reset_omax, nimp);
-        launch_n_raw(k_fine_keys<R>, N_, view(), keys_by_gid_, cell_cnt_, pf_tmp_, cpk_tmp_);
+        if (!begun) launch_small(k_sort_begin, nimp);
+        launch_n_raw(k_fine_keys<R>, N_, view(), key_rank_, cell_cnt_, pf_tmp_, cpk_tmp_);
         prof_begin();
-        launches_ += radix_sort_pairs(keys_by_gid_, nullptr, skeys_, sgid_, tkeys_, tgid_, G_,
-                                      key_bits(), scratch_, st_);
         launches_ += exclusive_scan_i32(cell_cnt_, cell_cnt_, C_ + 1, scratch_, st_);
         prof_end();
         int64_t n_new = N_;
@@ -2357,25 +2364,35 @@ public:
             n_new = flags_h_[2];
         }
         const int alt = cur_ ^ 1;
+        {
+            const unsigned nb = blocks_of(N_);
+            prof_begin();
+            k_place<<<nb + blocks_of(std::max(nimp, 1)), 256, 0, st_>>>(N_, key_rank_, gid_[cur_], cell_cnt_, slot_, tab_d_,
+                                                                      nimp, nb, rounds ? 1 : 0, flags_d_);
+            launched((const void*)k_place);
+            prof_end();
+            launches_++;
+        }
         if (n_new > 0) {
-            launch_n_raw(k_make_src, n_new, n_new, (const int32_t*)sgid_, (const int32_t*)pos_of_gid_, src_);
             GatherCols g{};
             for (int c = 0; c < kND; c++) { g.din[c] = dcol_[cur_][c]; g.dout[c] = dcol_[alt][c]; }
             g.nr = kNR;
             for (int c = 0; c < kNR; c++) { g.rin[c] = rcol_[cur_][c]; g.rout[c] = rcol_[alt][c]; }
+            static_assert(RC_MASS == 4, "the gather takes the mass column for the density records");
             g.b_in[0] = mat_[cur_]; g.b_out[0] = mat_[alt];
             g.b_in[1] = fixed_[cur_]; g.b_out[1] = fixed_[alt];
             g.imp_in = impc_[cur_]; g.imp_out = impc_[alt];
-            g.gid_in = gid_[cur_]; g.gid_out = gid_[alt];
+            g.gid_out = gid_[alt];
             g.pf_in = pf_tmp_; g.pf_out = pf_;
             g.cpk_in = cpk_tmp_; g.cpk_out = cpk_;
             g.lf_out = lf_; g.imps = tab_d_;
-            launch_n_raw(k_gather<R>, n_new, n_new, (const int32_t*)src_, g);
+            g.key_rank = key_rank_; g.slot = slot_; g.cell_ptr = cell_cnt_;
+            g.pos_of_gid = pos_of_gid_; g.pk_out = pk_; g.xcnt = xcnt_; g.refbin = refbin_;
+            g.rounds = rounds ? 1 : 0;
+            launch_n_raw(k_gather<R>, n_new, n_new, g);
         }
         cur_ = alt;
         N_ = n_new;
-        launch_n_raw(k_post_sort<R>, N_, view(), pos_of_gid_);
-        launch_small(k_impact_ranges, nimp, (const int32_t*)cell_cnt_);
         cls(keep_cls);
         grid_valid_ = true;
     }
@@ -2383,18 +2400,23 @@ public:
     // Neighbour lists.  The step uses one superset list (see k_list_thread);
     // capacity overflow is handled by the consumers' traversal fallback, and
     // the capacity grows for later steps when host_check reads the overflow.
+    // fresh: the sort just made has cleared the flags and the extra lists.
     template <int KIND>
-    void build_list(bool host_check) {
+    void build_list(bool host_check, bool fresh = false) {
         if (N_ <= 0) return;
         const int nimp = (int)imp_.size();
         const int keep = cur_cls_;
-        cls(KC_OTHER);
-        launch_small(k_impact_reset_slack, nimp);
-        cls(keep);
+        if (!fresh) {
+            cls(KC_OTHER);
+            launch_small(k_impact_reset_slack, nimp);
+            cls(keep);
+        }
         for (int attempt = 0; attempt < 8; attempt++) {
-            DSPH_CUDA(cudaMemsetAsync(flags_d_, 0, sizeof(int32_t), st_));
-            DSPH_CUDA(cudaMemsetAsync(flags_d_ + 2, 0, sizeof(int32_t), st_));
-            DSPH_CUDA(cudaMemsetAsync(xcnt_, 0, sizeof(int32_t) * N_, st_));
+            if (!fresh || attempt > 0) {
+                DSPH_CUDA(cudaMemsetAsync(flags_d_, 0, sizeof(int32_t), st_));
+                DSPH_CUDA(cudaMemsetAsync(flags_d_ + 2, 0, sizeof(int32_t), st_));
+                DSPH_CUDA(cudaMemsetAsync(xcnt_, 0, sizeof(int32_t) * N_, st_));
+            }
             if (list_mode_ == 1 && !levels_active_) {  // graded impacts: the per-thread builder
                 DSPH_CUDA(cudaMemsetAsync(ntask_, 0, sizeof(int32_t), st_));
                 launch_n_raw(k_column_tasks<R>, N_, view(), tasks_, ntask_);
@@ -2413,9 +2435,6 @@ public:
             } else {
                 launch_list_thread(0);
             }
-            cls(KC_OTHER);
-            launch_n_raw(k_sort_extra<R>, N_, view(), 0);
-            cls(keep);
             if (!host_check) return;
             DSPH_CUDA(cudaMemcpyAsync(flags_h_, flags_d_, sizeof(int32_t), cudaMemcpyDeviceToHost, st_));
             DSPH_CUDA(cudaStreamSynchronize(st_));
@@ -2451,10 +2470,7 @@ public:
         if (N_ <= 0 || list_mode_ != 0) return;  // other builders: the consumers' fallback
         const int keep = cur_cls_;
         cls(KC_LIST_FORCE);
-        launch_n(k_refresh_begin<R>, N_);
-        launch_list_thread(1);
-        launch_n_raw(k_sort_extra<R>, N_, view(), 1);
-        launch_small(k_impact_end_refresh, (int)imp_.size());
+        launch_list_thread(1);  // k_ref_bins has emptied the extra lists; k_eos ends the refresh
         cls(keep);
     }
 
@@ -2481,16 +2497,13 @@ public:
         launches_++;
     }
 
+    // Density rounds after a sort made for them (its first round's grid and
+    // bins are in place).
     void density_rounds(int iters, bool host_sync) {
         const int nimp = (int)imp_.size();
-        cls(KC_GRID);
-        launch_small(k_impact_begin_round, nimp, 2);
         for (int round = 0; round < 4; round++) {
             cls(KC_GRID);
-            if (round > 0) launch_small(k_impact_begin_round, nimp, 0);  // max h carried over
-            else hmax_pass(0);
-            launch_small(k_ref_grid, nimp);
-            launch_n(k_ref_bins<R>, N_);
+            if (round > 0) launch_n_raw(k_ref_bins<R>, N_, view(), 0);
             cls(KC_DENSITY);
             if (iters > 0) {  // also reduces the new max h
                 if (levels_active_) launch_n_raw(k_density<R, true>, N_, view(), iters);
@@ -2499,38 +2512,39 @@ public:
             }
             else hmax_pass(1);
             cls(KC_GRID);
-            DSPH_CUDA(cudaMemsetAsync(flags_d_ + 1, 0, sizeof(int32_t), st_));
-            launch_small(k_round_check, nimp, flags_d_);
-            if (host_sync) {
+            if (host_sync) DSPH_CUDA(cudaMemsetAsync(flags_d_ + 1, 0, sizeof(int32_t), st_));
+            launch_small(k_round, nimp, flags_d_, round < 3 ? (int)kRoundNext : (int)kRoundFinal);
+            if (host_sync && round < 3) {
                 DSPH_CUDA(cudaMemcpyAsync(flags_h_ + 1, flags_d_ + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st_));
                 DSPH_CUDA(cudaStreamSynchronize(st_));
-                if (!flags_h_[1]) break;
+                if (!flags_h_[1]) {
+                    launch_small(k_round, nimp, flags_d_, (int)kRoundOnlyFinal);
+                    break;
+                }
             }
         }
-        final_grid_build(true);
+        launch_n_raw(k_ref_bins<R>, N_, view(), host_sync || list_mode_ != 0 ? 0 : 1);
     }
 
-    // Reference grid and bins for the force pass; after_rounds: the max h is the
-    // one the last density pass reduced.
-    void final_grid_build(bool after_rounds = false) {
+    // Reference grid and bins of the current h, outside the rounds.
+    void final_grid_build() {
         const int nimp = (int)imp_.size();
         cls(KC_GRID);
-        launch_small(k_impact_begin_round, nimp, after_rounds ? 3 : 1);
-        if (!after_rounds) hmax_pass(0);
+        launch_small(k_impact_begin_round, nimp);
+        hmax_pass(0);
         launch_small(k_ref_grid, nimp);
-        launch_n(k_ref_bins<R>, N_);
+        launch_n_raw(k_ref_bins<R>, N_, view(), 0);
     }
 
     void forces(bool host_check) {
         if (host_check) refresh_list_if_needed();
         cls(KC_EOS);
-        launch_n(k_eos<R>, N_);
+        launch_eos(false);
         cls(KC_FORCE);
         launch_force();
     }
 
-    void dt_reduce() {
-        launch_small(k_dt_begin, (int)imp_.size());
+    void dt_reduce() {  // k_eos has reset the minimum
         launch_n(k_dt<R>, N_);
     }
 
@@ -2589,9 +2603,9 @@ public:
     int nsm_ = 148;
     uint32_t* cpk_ = nullptr;
     unsigned long long* refbin_ = nullptr;
-    int32_t* src_ = nullptr;
-    uint32_t *keys_by_gid_ = nullptr, *skeys_ = nullptr, *tkeys_ = nullptr;
-    int32_t *sgid_ = nullptr, *tgid_ = nullptr, *pos_of_gid_ = nullptr;
+    uint2* key_rank_ = nullptr;    // cell key and order of arrival, by current position
+    int2* slot_ = nullptr;         // (current position, id) by cell, in order of arrival
+    int32_t* pos_of_gid_ = nullptr;
     int32_t* cell_cnt_ = nullptr;
     int32_t* nbr_ = nullptr;
     int32_t* nbr_cnt_ = nullptr;

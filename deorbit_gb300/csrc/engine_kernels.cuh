@@ -621,9 +621,27 @@ __device__ __forceinline__ void walk_list_pairs(const int32_t* nbr, int64_t ls, 
 
 // ---------------------------------------------------------------- kernels
 
-// Kick (half step with the old acceleration) and drift (sph.hpp:360-361).
+// Start of a cell sort, per impact: the key pass reduces the largest offset and
+// the largest h, and the reference bins of the old order are void.
+__device__ __forceinline__ void sort_begin(ImpactD& I) {
+    I.omax_bits = 0u;
+    I.bins_ok = 0;
+    if (I.mask) I.hmax_bits = 0x3bc79ca10c924223ull;  // bits of 1e-30 (> 0)
+}
+static __global__ void k_sort_begin(ImpactD* imps, int nimp) {
+    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < nimp) sort_begin(imps[b]);
+}
+
+// Kick (half step with the old acceleration) and drift (sph.hpp:360-361); the
+// blocks past the particles' (from block nb) do sort_begin for the impacts.
 template <class R>
-static __global__ void k_kick_drift(View<R> v) {
+static __global__ void k_kick_drift(View<R> v, unsigned nb, int nimp) {
+    if (blockIdx.x >= nb) {
+        const int b = (blockIdx.x - nb) * blockDim.x + threadIdx.x;
+        if (b < nimp) sort_begin(v.imps[b]);
+        return;
+    }
     int64_t k = gtid();
     if (k >= v.n) return;
     const ImpactD& I = v.imps[v.imp[k]];
@@ -660,11 +678,9 @@ __device__ __forceinline__ int fine_cell(const ImpactD& I, int a, double c, floa
 // One particle's key, counts, offsets and packed cell; returns the bits of its
 // largest |offset| (ordered as the non-negative floats).
 template <class R>
-__device__ __forceinline__ unsigned int fine_keys_one(const View<R>& v, const ImpactD& I, int64_t k,
-                                                      uint32_t* keys_by_gid, int32_t* cell_count, float4* pf_out,
-                                                      uint32_t* cpk_out) {
+__device__ __forceinline__ unsigned int fine_keys_one(const View<R>& v, const ImpactD& I, int64_t k, uint2* key_rank,
+                                                      int32_t* cell_count, float4* pf_out, uint32_t* cpk_out) {
     const float h = (float)v.hh[k];  // loaded before the stores below
-    const int32_t gid = v.gid[k];
     float ox, oy, oz;
     int cx, cy, cz;
     int64_t key;
@@ -705,35 +721,66 @@ __device__ __forceinline__ unsigned int fine_keys_one(const View<R>& v, const Im
                   I.lev_nf[L][2] +
               ((cz >> L) - I.lev_lo[L][2]);
     }
-    keys_by_gid[gid] = (uint32_t)key;
-    atomicAdd(&cell_count[key], 1);
+    key_rank[k] = make_uint2((uint32_t)key, (uint32_t)atomicAdd(&cell_count[key], 1));
     pf_out[k] = make_float4(ox, oy, oz, h);
     cpk_out[k] = (uint32_t)cx | ((uint32_t)cy << 11) | ((uint32_t)cz << 22);
     return __float_as_uint(fmaxf(fmaxf(fabsf(ox), fabsf(oy)), fabsf(oz)));
 }
 
-// Traversal-cell key of every resident particle, scattered into gid order,
-// per-cell counts, and (in the current order, for the gather to carry) the
-// FP32 offset from the cell origin with h, the packed cell coordinates and the
-// per-impact largest |offset|.
+// Traversal-cell key of every resident particle with its order of arrival in
+// the cell, per-cell counts, and (in the current order, for the gather to carry)
+// the FP32 offset from the cell origin with h, the packed cell coordinates, the
+// per-impact largest |offset| and the largest h (masked impacts).
 template <class R>
-static __global__ void k_fine_keys(View<R> v, uint32_t* keys_by_gid, int32_t* cell_count, float4* pf_out,
+static __global__ void k_fine_keys(View<R> v, uint2* key_rank, int32_t* cell_count, float4* pf_out,
                                    uint32_t* cpk_out) {
     const int64_t k0 = gtid();
     const bool inb = k0 < v.n;
     const int64_t k = inb ? k0 : v.n - 1;
     ImpactD& I = v.imps[v.imp[k]];
-    const bool live = inb && I.alive;  // a dead impact's particles leave at this sort (key stays invalid)
+    const bool live = inb && I.alive;  // a dead impact's particles leave at this sort
     unsigned int om = 0u;
-    if (live) om = fine_keys_one(v, I, k, keys_by_gid, cell_count, pf_out, cpk_out);
+    if (live) om = fine_keys_one(v, I, k, key_rank, cell_count, pf_out, cpk_out);
+    else if (inb) key_rank[k] = make_uint2(kInvalidKey, 0u);
     block_atomic_ext<true>(&I.omax_bits, om, live);
+    block_atomic_ext<true>(&I.hmax_bits, dbits((double)v.hh[k]), live && I.mask);
 }
 
-static __global__ void k_make_src(int64_t n, const int32_t* sorted_gid, const int32_t* pos_of_gid,
-                           int32_t* src) {
-    int64_t k = gtid();
+// The cell sort proper.  Cells hold a handful of particles, so a particle's
+// place is its cell's start plus its rank by id among the cell's particles: it
+// first takes the slot of its arrival (this kernel), and the gather counts the
+// smaller ids of the cell (the order of arrival, which varies, drops out).
+// Against three 8-bit radix passes over (key, id): 1,048,576 particles 0.28 ->
+// 0.16 ms for keys, sort and gather, 6,000 particles 108 -> 38 us.
+// Blocks from nb on set up the impacts: sorted ranges and, with `rounds`, the
+// first density round's reference grid.
+__device__ __forceinline__ void impact_range(ImpactD& I, const int32_t* cell_ptr);
+__device__ __forceinline__ void ref_grid(ImpactD& I);
+__device__ __forceinline__ unsigned long long ref_bins(const ImpactD& I, double x, double y, double z);
+static __global__ void k_place(int64_t n, const uint2* key_rank, const int32_t* gid, const int32_t* cell_ptr, int2* slot,
+                               ImpactD* imps, int nimp, unsigned nb, int rounds, int32_t* flags) {
+    if (blockIdx.x >= nb) {
+        const int b = (blockIdx.x - nb) * blockDim.x + threadIdx.x;
+        if (b == 0) flags[0] = flags[2] = 0;
+        if (b >= nimp) return;
+        ImpactD& I = imps[b];
+        impact_range(I, cell_ptr);
+        if (I.mask) I.slack_flag = 0;
+        if (rounds) {
+            I.active = I.mask;
+            if (I.mask) {
+                I.rounds = 0;
+                I.bins_ok = 0;
+                ref_grid(I);
+            }
+        }
+        return;
+    }
+    const int64_t k = gtid();
     if (k >= n) return;
-    src[k] = pos_of_gid[sorted_gid[k]];
+    const uint2 kr = key_rank[k];
+    if (kr.x == kInvalidKey) return;
+    slot[cell_ptr[kr.x] + (int32_t)kr.y] = make_int2((int32_t)k, gid[k]);
 }
 
 // Gather of all carried columns into sorted order.
@@ -747,7 +794,6 @@ struct GatherCols {
     uint8_t* b_out[2];
     const uint16_t* imp_in;
     uint16_t* imp_out;
-    const int32_t* gid_in;
     int32_t* gid_out;
     const float4* pf_in;     // offsets + h and packed cells made by k_fine_keys
     float4* pf_out;
@@ -755,13 +801,26 @@ struct GatherCols {
     uint32_t* cpk_out;
     float4* lf_out;          // list frame, formed from the cell and the offset
     const ImpactD* imps;
+    const uint2* key_rank;   // of the current order
+    const int2* slot;        // (current position, id) by cell, in order of arrival
+    const int32_t* cell_ptr;
+    int32_t* pos_of_gid;     // inverse permutation
+    float2* pk_out;          // mixed form: (mass, packed cell) records of the density gathers
+    int32_t* xcnt;           // cleared for the list build
+    unsigned long long* refbin;  // bins of the first density round's reference grid (rounds)
+    int rounds;
 };
 
 template <class R>
-static __global__ void k_gather(int64_t n, const int32_t* src, GatherCols g) {
-    int64_t k = gtid();
-    if (k >= n) return;
-    int64_t s = src[k];
+static __global__ void k_gather(int64_t n, GatherCols g) {
+    int64_t at = gtid();
+    if (at >= n) return;
+    const int2 me = g.slot[at];
+    const int64_t s = me.x;
+    const uint32_t key = g.key_rank[s].x;
+    const int32_t cs = g.cell_ptr[key], ce = g.cell_ptr[key + 1];
+    int64_t k = cs;
+    for (int32_t q = cs; q < ce; q++) k += g.slot[q].y < me.y;
     // every load first, then every store: the column pointers may alias as far
     // as the compiler knows, so interleaved copies would wait for each load in turn
     double dv[7];
@@ -773,7 +832,7 @@ static __global__ void k_gather(int64_t n, const int32_t* src, GatherCols g) {
         if (c < g.nr) rv[c] = static_cast<const R*>(g.rin[c])[s];
     const uint8_t b0 = g.b_in[0][s], b1 = g.b_in[1][s];
     const uint16_t ib = g.imp_in[s];
-    const int32_t gid = g.gid_in[s];
+    const int32_t gid = me.y;
     const float4 p = g.pf_in[s];
     const uint32_t c = g.cpk_in[s];
 #pragma unroll
@@ -792,23 +851,14 @@ static __global__ void k_gather(int64_t n, const int32_t* src, GatherCols g) {
     const ImpactD& I = g.imps[ib];
     g.lf_out[k] = make_float4((float)(c & 2047u) * I.wf[0] + p.x, (float)((c >> 11) & 2047u) * I.wf[1] + p.y,
                               (float)(c >> 22) * I.wf[2] + p.z, p.w);
-}
-
-// After the gather: inverse permutation (gid -> sorted position) and, in the
-// mixed form, the (mass, packed cell) records of the density gathers.
-template <class R>
-static __global__ void k_post_sort(View<R> v, int32_t* pos_of_gid) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
-    pos_of_gid[v.gid[k]] = (int32_t)k;
-    if (sizeof(R) == 4) v.pk[k] = make_float2((float)v.mass[k], __uint_as_float(v.cpk[k]));
+    g.pos_of_gid[gid] = (int32_t)k;
+    g.xcnt[k] = 0;
+    if (sizeof(R) == 4) g.pk_out[k] = make_float2((float)rv[4], __uint_as_float(c));  // rv[4]: the mass
+    if (g.rounds && I.mask) g.refbin[k] = ref_bins(I, dv[0], dv[1], dv[2]);
 }
 
 // Per-impact sorted ranges from the cell pointer.
-static __global__ void k_impact_ranges(ImpactD* imps, int nimp, const int32_t* cell_ptr) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nimp) return;
-    ImpactD& I = imps[b];
+__device__ __forceinline__ void impact_range(ImpactD& I, const int32_t* cell_ptr) {
     if (!I.alive) { I.off = 0; I.n = 0; return; }
     int64_t s = cell_ptr[I.cell_base], e = cell_ptr[I.cell_base + I.ncells];
     I.off = s;
@@ -826,46 +876,19 @@ static __global__ void k_impact_ranges(ImpactD* imps, int nimp, const int32_t* c
     I.lmargin = 1.0e-6f * (cmax + 4.0f * I.hcap) + 1.0e-30f;
 }
 
-// Start of an on-device list rebuild: empty the extra lists of the impacts
-// whose h outgrew the slack.
-template <class R>
-static __global__ void k_refresh_begin(View<R> v) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
-    const ImpactD& I = v.imps[v.imp[k]];
-    if (I.mask && I.slack_flag) v.xcnt[k] = 0;
-}
-
-// End of an on-device list rebuild: the rebuilt lists cover the new h.
-static __global__ void k_impact_end_refresh(ImpactD* imps, int nimp) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < nimp && imps[b].mask) imps[b].slack_flag = 0;
-}
-
-// Phase flags: 0 = clear reductions for masked impacts.
+// A list rebuild outside a sort.
 static __global__ void k_impact_reset_slack(ImpactD* imps, int nimp) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < nimp && imps[b].mask) imps[b].slack_flag = 0;
 }
 
-// set_active: 2 first round of a step, 0 a later round, 1 a grid build outside
-// the rounds, 3 the grid build after the rounds.  The max h at a round's start
-// (and at the build after the rounds) is the max the previous round's density
-// pass reduced (h does not change in between); otherwise it is reduced anew.
-static __global__ void k_impact_begin_round(ImpactD* imps, int nimp, int set_active) {
+// A grid build outside the rounds: the max h is reduced anew (k_hmax).
+static __global__ void k_impact_begin_round(ImpactD* imps, int nimp) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nimp) return;
     ImpactD& I = imps[b];
-    if (set_active) {
-        I.active = I.mask;
-        if (set_active == 2 && I.mask) {
-            I.rounds = 0;
-            I.bins_ok = 0;
-        }
-    }
-    if (I.mask && I.active)
-        I.hmax_bits = (set_active == 0 || set_active == 3) ? I.hm_bits
-                                                           : 0x3bc79ca10c924223ull;  // bits of 1e-30 (> 0)
+    I.active = I.mask;
+    if (I.mask) I.hmax_bits = 0x3bc79ca10c924223ull;  // bits of 1e-30 (> 0)
 }
 
 template <class R>
@@ -879,11 +902,7 @@ static __global__ void k_hmax(View<R> v, int which) {
 }
 
 // Reference grid of an impact (sph.hpp:147-157): h_max -> nc, cw.
-static __global__ void k_ref_grid(ImpactD* imps, int nimp) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nimp) return;
-    ImpactD& I = imps[b];
-    if (!(I.mask && I.active)) return;
+__device__ __forceinline__ void ref_grid(ImpactD& I) {
     double hm = bitsd(I.hmax_bits);
     if (hm < 1e-30) hm = 1e-30;
     I.h_max = hm;
@@ -912,32 +931,50 @@ static __global__ void k_ref_grid(ImpactD* imps, int nimp) {
     I.hm_bits = 0x3bc79ca10c924223ull;
 }
 
+static __global__ void k_ref_grid(ImpactD* imps, int nimp) {
+    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < nimp && imps[b].mask && imps[b].active) ref_grid(imps[b]);
+}
+
+__device__ __forceinline__ unsigned long long ref_bins(const ImpactD& I, double x, double y, double z) {
+    return (unsigned long long)ref_bin(I, 0, x) | ((unsigned long long)ref_bin(I, 1, y) << 21) |
+           ((unsigned long long)ref_bin(I, 2, z) << 42);
+}
+
+// Bins of the reference grid where it changed; refresh: the lists of impacts
+// whose h outgrew the slack are rebuilt next, so their extra lists empty here.
 template <class R>
-static __global__ void k_ref_bins(View<R> v) {
+static __global__ void k_ref_bins(View<R> v, int refresh) {
     int64_t k = gtid();
     if (k >= v.n) return;
     const ImpactD& I = v.imps[v.imp[k]];
+    if (refresh && I.mask && I.slack_flag) v.xcnt[k] = 0;
     if (!(I.mask && I.active) || I.bins_ok) return;
-    unsigned long long b0 = (unsigned long long)ref_bin(I, 0, v.x[k]);
-    unsigned long long b1 = (unsigned long long)ref_bin(I, 1, v.y[k]);
-    unsigned long long b2 = (unsigned long long)ref_bin(I, 2, v.z[k]);
-    v.refbin[k] = b0 | (b1 << 21) | (b2 << 42);
+    v.refbin[k] = ref_bins(I, v.x[k], v.y[k], v.z[k]);
 }
 
-// End of an adaptive-h round (sph.hpp:203-205): keep going while max h grew > 2%.
-static __global__ void k_round_check(ImpactD* imps, int nimp, int32_t* flags) {
+// Between density passes (sph.hpp:203-205): an impact keeps going while its max
+// h grew > 2%.  done: a round has run -- judge it; next: the grid of the next
+// round for the impacts still going, from the max h that round's density pass
+// reduced; final: the grid after the rounds, for every masked impact.
+enum { kRoundNext = 0, kRoundFinal = 1, kRoundOnlyFinal = 2 };
+static __global__ void k_round(ImpactD* imps, int nimp, int32_t* flags, int mode) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nimp) return;
     ImpactD& I = imps[b];
-    if (!(I.mask && I.active)) return;
-    I.bins_ok = 1;  // this round's bins exist
-    I.rounds++;
-    double hm = bitsd(I.hm_bits);
-    if (hm < 1e-30) hm = 1e-30;
-    if (hm <= I.hmax0 * 1.02) {
-        I.active = 0;
-    } else {
-        atomicOr(&flags[1], 1);
+    if (!I.mask) return;
+    if (mode != kRoundOnlyFinal && I.active) {
+        I.bins_ok = 1;  // this round's bins exist
+        I.rounds++;
+        double hm = bitsd(I.hm_bits);
+        if (hm < 1e-30) hm = 1e-30;
+        if (hm <= I.hmax0 * 1.02) I.active = 0;
+        else atomicOr(&flags[1], 1);
+    }
+    if (mode != kRoundNext) I.active = 1;
+    if (I.active) {
+        I.hmax_bits = I.hm_bits;
+        ref_grid(I);
     }
 }
 
@@ -1492,13 +1529,9 @@ static __global__ void __launch_bounds__(256) k_list_wpp(View<R> v) {
     }
 }
 
-// Sort each particle's extra list (filled by atomics) into ascending order
-// (refresh != 0: only in impacts whose lists are being rebuilt).
+// A particle's extra list (filled by atomics) into ascending order.
 template <class R>
-static __global__ void k_sort_extra(View<R> v, int refresh) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
-    if (refresh && !v.imps[v.imp[k]].slack_flag) return;
+__device__ __forceinline__ void sort_extra(const View<R>& v, int64_t k) {
     const int c = min(v.xcnt[k], kExtraCap);
     if (c < 2) return;
     int32_t* a = v.xnbr + k;  // entry t at a[t * ls]
@@ -1667,11 +1700,21 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
 }
 
 // EOS + damage pre-pass (sph.hpp:261-275) and per-particle factors reused by
-// the pair loop.
+// the pair loop; the particle's extra list is put in order for it.  Blocks from
+// nb on: the impacts' CFL minimum is reset for k_finish, and (refreshed) lists
+// rebuilt since the density passes cover the new h.
 template <class R>
-static __global__ void k_eos(View<R> v) {
+static __global__ void k_eos(View<R> v, unsigned nb, int nimp, int refreshed) {
+    if (blockIdx.x >= nb) {
+        const int b = (blockIdx.x - nb) * blockDim.x + threadIdx.x;
+        if (b >= nimp || !v.imps[b].mask) return;
+        v.imps[b].dt_bits = 0x7ff0000000000000ull;  // +inf
+        if (refreshed) v.imps[b].slack_flag = 0;
+        return;
+    }
     int64_t k = gtid();
     if (k >= v.n) return;
+    sort_extra(v, k);
     const ImpactD& I = v.imps[v.imp[k]];
     if (!I.mask) return;
     const MatT<R> m = v.mats[v.mat[k]];
@@ -2104,11 +2147,8 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
 
 // Crack growth (sph.hpp:336-348); multi-flaw extension by gid.
 template <class R>
-static __global__ void k_damage(View<R> v) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
-    const ImpactD& I = v.imps[v.imp[k]];
-    if (!I.mask || !I.damage_on) return;
+__device__ __forceinline__ void damage_one(const View<R>& v, const ImpactD& I, int64_t k) {
+    if (!I.damage_on) return;
     const MatT<R>& m = v.mats[v.mat[k]];
     const R D = v.D[k];
     if (m.Emod <= R(0) || D >= R(1)) return;
@@ -2138,11 +2178,7 @@ static __global__ void k_damage(View<R> v) {
 // Second kick, trapezoidal u and S, u floor, yield (sph.hpp:365-376); the new
 // derivatives become the carried ones for the next step's trapezoid.
 template <class R>
-static __global__ void k_finish(View<R> v) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
-    const ImpactD& I = v.imps[v.imp[k]];
-    if (!I.mask) return;
+__device__ __forceinline__ void finish_one(const View<R>& v, const ImpactD& I, int64_t k) {
     const R dn = v.dudt_new[k];
     R dsn[6];
 #pragma unroll
@@ -2198,26 +2234,15 @@ static __global__ void k_adopt_derivatives(View<R> v) {
     for (int c = 0; c < 6; c++) v.dS[c][k] = v.dS_new[c][k];
 }
 
-static __global__ void k_dt_begin(ImpactD* imps, int nimp) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nimp) return;
-    if (imps[b].mask) imps[b].dt_bits = 0x7ff0000000000000ull;  // +inf
-}
-
 // CFL step (sph.hpp:350-355): per-impact min of cfl h / (csig (1 + alpha) + 1e-30).
 // The FP64 quotient is formed only where it can be the minimum: an FP32
 // estimate (within 3e-7 of it) is reduced over the warp first, and only lanes
 // within 1e-5 of the warp's smallest estimate -- which include the lane of the
 // exact minimum -- divide in FP64 (warps that straddle two impacts: all lanes).
+// Every thread of the block calls it.
 template <class R>
-static __global__ void k_dt(View<R> v) {
+__device__ __forceinline__ void dt_one(const View<R>& v, ImpactD& I, int ib, int64_t k, bool live) {
     const unsigned full = 0xffffffffu;
-    const int64_t k0 = gtid();
-    const bool inb = k0 < v.n;
-    const int64_t k = inb ? k0 : v.n - 1;
-    const int ib = v.imp[k];
-    ImpactD& I = v.imps[ib];
-    const bool live = inb && I.mask;
     const float qf = live ? (float)v.hh[k] / ((float)v.csig[k] * (1.0f + (float)I.alpha) + 1e-30f) : INFINITY;
     const bool uniform = __all_sync(full, ib == __shfl_sync(full, ib, 0));
     const float qmin = __uint_as_float(__reduce_min_sync(full, __float_as_uint(qf)));  // qf >= 0
@@ -2227,24 +2252,49 @@ static __global__ void k_dt(View<R> v) {
     block_atomic_ext<false>(&I.dt_bits, dbits(d), cand);
 }
 
+template <class R>
+static __global__ void k_dt(View<R> v) {
+    const int64_t k0 = gtid();
+    const int64_t k = k0 < v.n ? k0 : v.n - 1;
+    const int ib = v.imp[k];
+    ImpactD& I = v.imps[ib];
+    dt_one(v, I, ib, k, k0 < v.n && I.mask);
+}
+
+// The end of a step in one pass: crack growth, the second kick with the
+// trapezoids and the yield, and the next CFL step.
+template <class R>
+static __global__ void k_finish(View<R> v) {
+    const int64_t k0 = gtid();
+    const int64_t k = k0 < v.n ? k0 : v.n - 1;
+    const int ib = v.imp[k];
+    ImpactD& I = v.imps[ib];
+    const bool live = k0 < v.n && I.mask;
+    if (live) {
+        damage_one(v, I, k);
+        finish_one(v, I, k);
+    }
+    dt_one(v, I, ib, k, live);
+}
+
 // Device-side step control for batched runs: dt = min(CFL dt, t_end - t);
-// impacts at t_end drop out of the mask.
+// impacts at t_end drop out of the mask.  phase 0: before a step, 1: after one,
+// 2: between two.
 static __global__ void k_run_control(ImpactD* imps, int nimp, int phase) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nimp) return;
     ImpactD& I = imps[b];
     if (!I.alive) { I.mask = 0; return; }
-    if (phase == 0) {  // before a step
+    if (phase != 0 && I.mask) {  // after a step
+        I.t += I.dt;
+        I.nsteps++;
+    }
+    if (phase != 1) {  // before a step
         if (I.t_end > 0 && I.t >= I.t_end) { I.mask = 0; return; }
         if (I.max_steps > 0 && I.nsteps >= I.max_steps) { I.mask = 0; return; }
         double dt = bitsd(I.dt_bits);
         if (I.t_end > 0 && I.t + dt > I.t_end) dt = I.t_end - I.t;
         I.dt = dt;
-    } else {  // after a step
-        if (I.mask) {
-            I.t += I.dt;
-            I.nsteps++;
-        }
     }
 }
 

@@ -69,8 +69,19 @@ __global__ void k_scan_sums(int32_t* sums, int64_t nt) {
     }
 }
 
-__global__ void k_tile_scan(const int32_t* in, int32_t* out, int64_t n, const int32_t* offs) {
+// offs: the tiles' exclusive offsets, or (sums) the tiles' sums, which every
+// block adds up to its own -- a few thousand integers, cheaper than a launch.
+__global__ void k_tile_scan(const int32_t* in, int32_t* out, int64_t n, const int32_t* offs, int sums) {
     __shared__ int32_t ws[kScanThreads / 32];
+    int32_t before = 0;
+    if (sums) {
+        for (int64_t t = threadIdx.x; t < (int64_t)blockIdx.x; t += kScanThreads) before += offs[t];
+        int32_t tot;
+        block_exclusive_scan(before, ws, tot);
+        before = tot;
+    } else {
+        before = offs[blockIdx.x];
+    }
     int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kScanItems;
     int32_t v[kScanItems];
     int32_t s = 0;
@@ -80,7 +91,7 @@ __global__ void k_tile_scan(const int32_t* in, int32_t* out, int64_t n, const in
         s += v[i];
     }
     int32_t tot;
-    int32_t ex = block_exclusive_scan(s, ws, tot) + offs[blockIdx.x];
+    int32_t ex = block_exclusive_scan(s, ws, tot) + before;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         if (base + i < n) out[base + i] = ex;
@@ -89,8 +100,6 @@ __global__ void k_tile_scan(const int32_t* in, int32_t* out, int64_t n, const in
 }
 
 // ---- radix sort ------------------------------------------------------------
-// Items of a tile are striped: round r, thread t -> tile index r*256 + t, so
-// the stable order inside the tile is (round, warp, lane).
 
 __global__ void k_digit_hist(const uint32_t* keys, int64_t n, int shift, int32_t* hist,
                              int64_t ntiles) {
@@ -107,53 +116,57 @@ __global__ void k_digit_hist(const uint32_t* keys, int64_t n, int shift, int32_t
     hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void k_digit_scatter(const uint32_t* keys_in, const int32_t* vals_in,
-                                uint32_t* keys_out, int32_t* vals_out, int64_t n, int shift,
-                                const int32_t* offs, int64_t ntiles) {
+// Items of a tile: warp w owns 256 consecutive ones, in 8 rounds of 32, so the
+// stable order inside the tile is (warp, round, lane).  A warp ranks its items
+// against its own counters without block barriers; one prefix over the warps per
+// digit then places them (three barriers a tile instead of five a round).
+__global__ void __launch_bounds__(kScanThreads) k_digit_scatter(const uint32_t* keys_in, const int32_t* vals_in,
+                                                                uint32_t* keys_out, int32_t* vals_out, int64_t n,
+                                                                int shift, const int32_t* offs, int64_t ntiles) {
     constexpr int W = kScanThreads / 32;
     __shared__ int32_t cnt[W][256];
-    __shared__ int32_t running[256];
-    __shared__ int32_t base_off[256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    running[tid] = 0;
-    base_off[tid] = offs[(int64_t)tid * ntiles + blockIdx.x];
-    const int64_t tbase = (int64_t)blockIdx.x * kTile;
-    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int w = 0; w < W; w++) cnt[w][tid] = 0;
+    const int32_t base_off = offs[(int64_t)tid * ntiles + blockIdx.x];
+    const int64_t base = (int64_t)blockIdx.x * kTile + warp * (32 * kScanItems) + lane;
+    uint32_t key[kScanItems];
+    int32_t val[kScanItems], rank[kScanItems];
+#pragma unroll
     for (int r = 0; r < kScanItems; r++) {
-        int64_t i = tbase + r * kScanThreads + tid;
-        bool valid = i < n;
-        uint32_t key = valid ? keys_in[i] : 0u;
-        int32_t val = valid ? (vals_in ? vals_in[i] : (int32_t)i) : 0;
-        int d = valid ? (int)((key >> shift) & 255u) : 256;
+        const int64_t i = base + r * 32;
+        key[r] = i < n ? keys_in[i] : 0u;
+        val[r] = i < n ? (vals_in ? vals_in[i] : (int32_t)i) : 0;
+    }
+    __syncthreads();
+    const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-        for (int w = 0; w < W; w++) cnt[w][tid] = 0;
-        __syncthreads();
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        int wrank = __popc(peers & lt);
-        bool leader = (peers & lt) == 0u;
-        if (valid && leader) cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        // exclusive prefix over warps for digit tid; round total
-        int32_t acc = 0;
+    for (int r = 0; r < kScanItems; r++) {
+        const bool valid = base + r * 32 < n;
+        const int d = valid ? (int)((key[r] >> shift) & 255u) : 256;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        rank[r] = valid ? cnt[warp][d] + __popc(peers & lt) : 0;
+        __syncwarp();
+        if (valid && (peers & lt) == 0u) cnt[warp][d] += __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    int32_t acc = base_off;
 #pragma unroll
-        for (int w = 0; w < W; w++) {
-            int32_t c = cnt[w][tid];
-            cnt[w][tid] = acc;
-            acc += c;
-        }
-        __syncthreads();
-        if (valid) {
-            int32_t pos = base_off[d] + running[d] + cnt[warp][d] + wrank;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-        }
-        __syncthreads();
-        running[tid] += acc;
-        __syncthreads();
+    for (int w = 0; w < W; w++) {
+        const int32_t c = cnt[w][tid];
+        cnt[w][tid] = acc;
+        acc += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kScanItems; r++) {
+        if (base + r * 32 >= n) continue;
+        const int32_t pos = cnt[warp][(key[r] >> shift) & 255u] + rank[r];
+        keys_out[pos] = key[r];
+        vals_out[pos] = val[r];
     }
 }
-
-
 
 }  // namespace
 
@@ -163,9 +176,12 @@ int exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, void* scratch
     int64_t nt = tiles_of(n);
     int32_t* sums = static_cast<int32_t*>(scratch);
     k_tile_sums<<<(unsigned)nt, kScanThreads, 0, st>>>(in, n, sums);
-    k_scan_sums<<<1, kScanThreads, 0, st>>>(sums, nt);
-    k_tile_scan<<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, sums);
-    return 3;
+    // the blocks' own additions grow as nt^2: 4096 tiles (8.4 M values) cost about
+    // what the separate launch over the sums does
+    const bool direct = nt <= 4096;
+    if (!direct) k_scan_sums<<<1, kScanThreads, 0, st>>>(sums, nt);
+    k_tile_scan<<<(unsigned)nt, kScanThreads, 0, st>>>(in, out, n, sums, direct ? 1 : 0);
+    return direct ? 2 : 3;
 }
 
 int radix_sort_pairs(const uint32_t* keys_in, const int32_t* vals_in, uint32_t* keys_out,

@@ -268,8 +268,8 @@ int sph_debug_flaws(sph_ctx* ctx, int32_t impact, int64_t* ptr, double* eps, int
  * perm[n] (device): particle indices ordered by (cell, index); cell_start
  * [ncells+1] (device): first sorted position of each cell, cell_start[ncells]
  * = n.  stream is a cudaStream_t (NULL: the legacy default stream); the call
- * returns when the result is complete.  Scratch is taken with
- * cudaMallocAsync on the stream and released before returning.
+ * returns when the result is complete.  Scratch comes, stream-ordered, from
+ * a pool of the library that keeps at most 64 MiB a device between calls.
  * SPH_ERR_ARG when a key is out of range (outputs then undefined). */
 int sph_cell_sort(const uint32_t* keys, int64_t n, int64_t ncells, int32_t* perm,
                   int32_t* cell_start, void* stream);
