@@ -38,6 +38,11 @@ __device__ __forceinline__ float rsqrt_(float x) { return sqrtf(x); }
 // integer pipes: fp64_int.cuh).
 __device__ __forceinline__ float pair_div(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double pair_div(double a, double b) { return fi::div(a, b); }
+// a b and a b + c with their roundings fixed in the source (never fused further, always fused)
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return fma(a, b, c); }
 // a / b of per-particle work: IEEE in both types
 __device__ __forceinline__ float rdiv(float a, float b) { return a / b; }
 __device__ __forceinline__ double rdiv(double a, double b) { return fi::div(a, b); }

@@ -1610,6 +1610,14 @@ private:
             if (h.used && h.alive && (h.per[0] | h.per[1] | h.per[2])) return true;
         return false;
     }
+    // Runs of few particles take eight lanes to a particle in the list build and
+    // the mixed form's pair passes (same results): below these counts the
+    // thread-per-particle kernels leave SMs with too few warps to cover a pair's
+    // loads.  Thread / lanes, us: 5,864 particles list 98 / 46, density 47 / 18,
+    // force 69 / 23; 22,040: 94 / 52, 47 / 31, 66 / 50; 39,464: 98 / 86, 45 / 42,
+    // 67 / 74; 64,280: 109 / 95, 49 / 61, 78 / 111; 85,544: 117 / 121 (list).
+    static constexpr int64_t kFewParticles = 32768, kFewForLists = 65536;
+    bool few_particles() const { return sizeof(R) == 4 && N_ <= kFewParticles && !levels_active_ && !any_periodic(); }
     void launch_force() {
         if (N_ <= 0) return;
         prof_begin();
@@ -1632,6 +1640,11 @@ private:
         } else if (!done && any_periodic()) {
             k_force<R, 0, 0, false, false, true><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
             launched((const void*)k_force<R, 0, 0, false, false, true>);
+        } else if (!done && few_particles()) {
+            if constexpr (sizeof(R) == 4) {
+                k_force<R, 0, 0, false, false, false, 8><<<(unsigned)((8 * N_ + 127) / 128), 128, 0, st_>>>(view(), wait_err_d_);
+                launched((const void*)k_force<R, 0, 0, false, false, false, 8>);
+            }
         } else if (!done) {  // no resident impact is periodic: pair loop without minimum image
             k_force<R, 0, 0, false, false, false><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
             launched((const void*)k_force<R, 0, 0, false, false, false>);
@@ -2454,6 +2467,9 @@ public:
         } else if (any_periodic()) {
             k_list_thread<R, false, true><<<(unsigned)((N_ + bs - 1) / bs), bs, 0, st_>>>(view(), refresh);
             launched((const void*)k_list_thread<R, false, true>);
+        } else if (N_ <= kFewForLists) {
+            k_list_group<R, 8><<<blocks_of(8 * N_), 256, 0, st_>>>(view(), refresh);
+            launched((const void*)k_list_group<R, 8>);
         } else {
             k_list_thread<R, false, false><<<(unsigned)((N_ + bs - 1) / bs), bs, 0, st_>>>(view(), refresh);
             launched((const void*)k_list_thread<R, false, false>);
@@ -2508,6 +2524,9 @@ public:
             if (iters > 0) {  // also reduces the new max h
                 if (levels_active_) launch_n_raw(k_density<R, true>, N_, view(), iters);
                 else if (any_periodic()) launch_n_raw(k_density<R, false, true>, N_, view(), iters);
+                else if (few_particles()) {
+                    if constexpr (sizeof(R) == 4) launch_n_raw(k_density<R, false, false, 8>, 8 * N_, view(), iters);
+                }
                 else launch_n_raw(k_density<R, false, false>, N_, view(), iters);
             }
             else hmax_pass(1);

@@ -1243,6 +1243,109 @@ static __global__ void k_list_thread(View<R> v, int refresh) {
     }
 }
 
+// The list build with G lanes to a particle (non-periodic impacts on one grid):
+// a column's candidates are tested 2 G at a time and the hits appended in
+// candidate order by a ballot, so the lists are k_list_thread's entry for entry.
+// A run of few particles leaves that kernel's warps waiting on one candidate
+// pair after another; here the same waits cover eight times as many.
+template <class R, int G>
+static __global__ void __launch_bounds__(256) k_list_group(View<R> v, int refresh) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
+    const int64_t k0 = gtid() / G;
+    const bool inb = k0 < v.n;
+    const int64_t k = inb ? k0 : v.n - 1;
+    const int ib = v.imp[k];
+    const ImpactD& I = v.imps[ib];
+    const bool wanted = I.mask && (!refresh || I.slack_flag);
+    const bool one_impact = __all_sync(full, ib == __shfl_sync(full, ib, 0));
+    if (!one_impact) {
+        if (inb && wanted && g == 0) list_one<R, false, false>(v, I, k);
+        return;
+    }
+    if (!wanted) return;  // warp-uniform: one impact
+    const float4 pi = v.pf[k];
+    const uint32_t ci = v.cpk[k];
+    const float4 li = v.lf[k];
+    const float m = (sizeof(R) == 8 ? I.margin : 0.0f) + I.lmargin;
+    const float sl = 1.0f + I.slack;
+    const float ri = 2.0f * pi.w * sl + m;
+    const float ri2 = ri * ri;
+    const float Rs = ri + m;
+    const float R2 = Rs * Rs;
+    int cnt = 0;
+    const int cap = v.cap;
+    int32_t* out = v.nbr + 4 * k;  // entry t at out[nbr_slot(t, ls)]
+    const unsigned below = (1u << g) - 1u;
+    auto take = [&](bool hit, int32_t j, float4 lj, float r2) {  // the whole warp
+        const unsigned hits = (__ballot_sync(full, hit) >> first) & ((1u << G) - 1u);
+        if (hit) {
+            const int at = cnt + __popc(hits & below);
+            if (at < cap) out[nbr_slot(at, v.ls)] = j;
+            const float rj = 2.0f * lj.w * sl + m;
+            const float rb = (pi.w + lj.w) * sl + m;
+            if (!(r2 < rj * rj) && r2 < rb * rb) {
+                const int slot = atomicAdd(&v.xcnt[j], 1);
+                if (slot < kExtraCap) v.xnbr[(int64_t)slot * v.ls + j] = (int32_t)k;
+            }
+        }
+        cnt += __popc(hits);
+    };
+    int c[3];
+    unpack_cell(ci, c[0], c[1], c[2]);
+    // ranges and chords as in k_list_thread
+    const float w0 = I.wf[0], w1 = I.wf[1];
+    const float iw0 = I.iwf[0], iw1 = I.iwf[1], iw2 = I.iwf[2];
+    const int nf0 = I.nf[0], nf1 = I.nf[1], nf2 = I.nf[2];
+    constexpr float kWiden = 1.0e-5f;
+    int lo0 = c[0] + (int)floorf((pi.x - Rs) * iw0 - kWiden), hi0 = c[0] + (int)floorf((pi.x + Rs) * iw0 + kWiden);
+    int lo1 = c[1] + (int)floorf((pi.y - Rs) * iw1 - kWiden), hi1 = c[1] + (int)floorf((pi.y + Rs) * iw1 + kWiden);
+    lo0 = lo0 < 0 ? 0 : (lo0 > nf0 - 1 ? nf0 - 1 : lo0);
+    hi0 = hi0 < 0 ? 0 : (hi0 > nf0 - 1 ? nf0 - 1 : hi0);
+    lo1 = lo1 < 0 ? 0 : (lo1 > nf1 - 1 ? nf1 - 1 : lo1);
+    hi1 = hi1 < 0 ? 0 : (hi1 > nf1 - 1 ? nf1 - 1 : hi1);
+    const int ulo0 = __reduce_min_sync(full, inb ? lo0 : INT_MAX), uhi0 = __reduce_max_sync(full, inb ? hi0 : INT_MIN);
+    const int ulo1 = __reduce_min_sync(full, inb ? lo1 : INT_MAX), uhi1 = __reduce_max_sync(full, inb ? hi1 : INT_MIN);
+    for (int ix = ulo0; ix <= uhi0; ix++) {
+        const float xa = (float)(ix - c[0]) * w0 - pi.x;
+        float bx = xa > 0.0f ? xa : (xa + w0 < 0.0f ? -(xa + w0) : 0.0f);
+        if (ix == 0 || ix == nf0 - 1) bx = 0.0f;
+        const bool in_x = inb && ix >= lo0 && ix <= hi0;
+        for (int iy = ulo1; iy <= uhi1; iy++) {
+            const float ya = (float)(iy - c[1]) * w1 - pi.y;
+            float by = ya > 0.0f ? ya : (ya + w1 < 0.0f ? -(ya + w1) : 0.0f);
+            if (iy == 0 || iy == nf1 - 1) by = 0.0f;
+            const float d2 = bx * bx + by * by;
+            int32_t s = 0, len = 0;
+            if (in_x && iy >= lo1 && iy <= hi1 && d2 < R2) {
+                const float q = R2 - d2;
+                const float hz = q * rsqrtf(q) * (1.0f + 1.0e-6f);  // hardware 1/sqrt (2 ulp), widened
+                int zl = c[2] + (int)floorf((pi.z - hz) * iw2 - kWiden);
+                int zh = c[2] + (int)floorf((pi.z + hz) * iw2 + kWiden);
+                zl = zl < 0 ? 0 : (zl > nf2 - 1 ? nf2 - 1 : zl);
+                zh = zh < 0 ? 0 : (zh > nf2 - 1 ? nf2 - 1 : zh);
+                const int64_t colbase = I.cell_base + ((int64_t)ix * nf1 + iy) * nf2;
+                s = v.cell_ptr[colbase + zl];
+                len = v.cell_ptr[colbase + zh + 1] - s;
+            }
+            const int maxlen = __reduce_max_sync(full, len);
+            for (int t = 0; t < maxlen; t += 2 * G) {
+                const bool ok0 = t + g < len, ok1 = t + G + g < len;
+                const int32_t j0 = ok0 ? s + t + g : (int32_t)k, j1 = ok1 ? s + t + G + g : (int32_t)k;
+                const float4 l0 = v.lf[j0], l1 = v.lf[j1];
+                const float r20 = list_r2(li, l0), r21 = list_r2(li, l1);
+                take(ok0 && r20 < ri2, j0, l0, r20);
+                take(ok1 && r21 < ri2, j1, l1, r21);
+            }
+        }
+    }
+    if (inb && g == 0) {
+        v.nbr_cnt[k] = cnt;
+        v.hlist[k] = pi.w;
+        if (cnt > cap) atomicMax(&v.flags[0], cnt);
+    }
+}
+
 // Work list for the warp-converged list build: one task per run of up to 32
 // consecutive sorted particles inside one traversal-cell column of one impact.
 template <class R>
@@ -1606,12 +1709,19 @@ __device__ __forceinline__ bool list_covers(const View<R>& v, const ImpactD& I, 
 // compensated sum in the mixed form.  An iteration reads only the particle's
 // own h and the neighbours' positions and masses, so running the iterations
 // back to back per particle gives the same result as one launch per iteration.
-template <class R, bool LV = false, bool PER = true>
+// G > 1 (mixed form, few particles): G lanes to a particle evaluate G entries at
+// once; every lane then adds them in list order, so the sums are the same.
+template <class R, bool LV = false, bool PER = true, int G = 1>
 static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(View<R> v, int iters) {
-    int64_t k = gtid();
-    if (k >= v.n) return;
+    static_assert(G == 1 || (sizeof(R) == 4 && !LV && !PER), "lane groups: mixed form, one grid, no periodic axis");
+    int64_t k = gtid() / G;
+    bool act = k < v.n;
+    if (G == 1 && !act) return;
+    if (!act) k = v.n - 1;
     ImpactD& I = v.imps[v.imp[k]];
-    if (!(I.mask && I.active)) return;
+    act = act && I.mask && I.active;
+    if (G == 1 && !act) return;
+    [[maybe_unused]] const int g = threadIdx.x & (G - 1);
     R hi = v.hh[k];
     const float4 pi = v.pf[k];
     const uint32_t ci = v.cpk[k];
@@ -1663,7 +1773,36 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
                 sum.add((R)w_mixed(j, v.pf[j], v.pk[j]));
             }
         };
-        if (list_covers(v, I, k, (float)hi)) {
+        if constexpr (G > 1) {
+            const unsigned full = 0xffffffffu;
+            const bool covers = act && list_covers(v, I, k, (float)hi);
+            const int cnt = covers ? v.nbr_cnt[k] : 0;
+            const int most = __reduce_max_sync(full, cnt);
+            const int32_t* nb = v.nbr + 4 * k;
+            for (int t = 0; t < most; t += 2 * G) {
+                const bool ok0 = t + g < cnt, ok1 = t + G + g < cnt;
+                const int32_t j0 = ok0 ? nb[nbr_slot(t + g, v.ls)] : (int32_t)k;
+                const int32_t j1 = ok1 ? nb[nbr_slot(t + G + g, v.ls)] : (int32_t)k;
+                const float4 p0 = v.pf[j0], p1 = v.pf[j1];
+                const float2 m0 = v.pk[j0], m1 = v.pk[j1];
+                const float w0 = w_mixed(j0, p0, m0), w1 = w_mixed(j1, p1, m1);
+#pragma unroll
+                for (int i = 0; i < G; i++) {
+                    const float w = __shfl_sync(full, w0, i, G);
+                    if (t + i < cnt) sum.add((R)w);
+                }
+#pragma unroll
+                for (int i = 0; i < G; i++) {
+                    const float w = __shfl_sync(full, w1, i, G);
+                    if (t + G + i < cnt) sum.add((R)w);
+                }
+            }
+            if (act && !covers) {  // every lane of the group walks the cells itself
+                const float hf = (float)hi;
+                traverse<R, LV>(v, I, pi, ci, 2.0f * hf * 1.0001f + 2.0f * I.margin + 1e-6f * hf,
+                         [&](int32_t j, float, float, float) { body(j); });
+            }
+        } else if (list_covers(v, I, k, (float)hi)) {
             const int cnt = v.nbr_cnt[k];
             if constexpr (sizeof(R) == 4) {
                 // two entries per trip: both loads in flight, summed in list order
@@ -1687,12 +1826,14 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
         rho_lo = rho > R(1e-30) ? sum.low() : R(0);
         hi = rmin(R(2) * h0, rmax(R(0.5) * h0, (R)I.eta * rcbrt(rdiv(mass_k, rho))));
     }
+    if (G > 1 && !act) return;
+    impact_atomic_max(&I.hm_bits, (double)hi);  // the round's new max h
+    if (G > 1 && g != 0) return;
     v.rho[k] = rho;
     v.rho_lo[k] = rho_lo;
     v.hh[k] = hi;
     v.pf[k].w = (float)hi;
     v.lf[k].w = (float)hi;
-    impact_atomic_max(&I.hm_bits, (double)hi);  // the round's new max h
     if (!((float)hi <= v.hlist[k] * (1.0f + I.slack) * 0.99999f)) {
         atomicOr(&I.slack_flag, 1);
         atomicOr(&v.flags[2], 1);
@@ -1812,18 +1953,29 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // ASYNC selects the copy engine of the staging: false = one bulk copy per
 // entry (cp.async.bulk, TMA), true = six 16-byte cp.async per entry (the load
 // path through L1, completion tracked by cp.async.mbarrier.arrive).
-template <class R, int SE = 0, int SS = 0, bool ASYNC = false, bool LV = false, bool PER = true>
+// NG = 8 (mixed form, few particles): eight lanes to a particle evaluate eight
+// entries at once and leave their terms in shared memory; seven of them then
+// add one pair of the sums each, entry by entry in list order, so the sums are
+// the same bit for bit.
+template <class R, int SE = 0, int SS = 0, bool ASYNC = false, bool LV = false, bool PER = true, int NG = 1>
 static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(View<R> v, int32_t* wait_err) {
     using Acc = AccT<R>;
     constexpr bool kStaged = SS > 0 && sizeof(R) == 4;
-    int64_t k = gtid();
+    static_assert(NG == 1 || (NG == 8 && sizeof(R) == 4 && !kStaged && !LV && !PER),
+                  "lane groups: mixed form, one grid, no periodic axis");
+    constexpr int kTerms = 7;  // per entry: four packed rows of L, L22, (ax, ay), (az, du)
+    __shared__ float4 terms[NG > 1 ? 128 * kTerms : 1];
+    [[maybe_unused]] const int g = threadIdx.x & (NG - 1);
+    [[maybe_unused]] float4* const mine = terms + (NG > 1 ? threadIdx.x * kTerms : 0);
+    [[maybe_unused]] const float4* const group = terms + (NG > 1 ? (threadIdx.x - g) * kTerms : 0);
+    int64_t k = gtid() / NG;
     bool live = k < v.n;
-    if constexpr (!kStaged) {
+    if constexpr (!kStaged && NG == 1) {
         if (!live) return;
     }
-    if (!live) k = v.n - 1;  // staged: every lane of the warp takes part in the barrier phases
+    if (!live) k = v.n - 1;  // staged, grouped: every lane of the warp takes part in the barrier phases
     const ImpactD& I = v.imps[v.imp[k]];
-    if constexpr (!kStaged) {
+    if constexpr (!kStaged && NG == 1) {
         if (!I.mask) return;
     }
     live = live && I.mask;
@@ -1888,11 +2040,19 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
         if (strength) {  // Vj (v_j - v_i) (x) grad W
             const float2 exy = mul2(vxy, f2(-Vj));
             const float ez = -vz * Vj;
-            Lp0 = fma2(f2(exy.x), gxy, Lp0);
-            Lp1 = fma2(f2(exy.y), gxy, Lp1);
-            Lp2 = fma2(f2(ez), gxy, Lp2);
-            Lpz = fma2(exy, f2(gz), Lpz);
-            Lp22 = fmaf(ez, gz, Lp22);
+            if constexpr (NG > 1) {
+                mine[0] = make_float4(exy.x, exy.x, gxy.x, gxy.y);
+                mine[1] = make_float4(exy.y, exy.y, gxy.x, gxy.y);
+                mine[2] = make_float4(ez, ez, gxy.x, gxy.y);
+                mine[3] = make_float4(exy.x, exy.y, gz, gz);
+                mine[4] = make_float4(ez, 0.0f, gz, 0.0f);
+            } else {
+                Lp0 = fma2(f2(exy.x), gxy, Lp0);
+                Lp1 = fma2(f2(exy.y), gxy, Lp1);
+                Lp2 = fma2(f2(ez), gxy, Lp2);
+                Lpz = fma2(exy, f2(gz), Lpz);
+                Lp22 = fmaf(ez, gz, Lp22);
+            }
         }
         const float dvr = vxy.x * dx + vxy.y * dy + vz * dz;
         float Pij = 0.0f;
@@ -1920,13 +2080,19 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
         const float2 stxy = fma2(oth, f2(dsj), mul2(own, f2((float)dsri)));
         const float stz = ((float)sxz * gxy.x + (float)syz * gxy.y + (float)szz * gz) * (float)dsri +
                           (fb.z * gxy.x + fb.w * gxy.y + fc.z * gz) * dsj;
-        kxy.add(fma2(gxy, f2(-mm), mul2(stxy, f2(mj))));
+        const float2 axy = fma2(gxy, f2(-mm), mul2(stxy, f2(mj)));
+        if constexpr (NG == 1) kxy.add(axy);
         if (alpha_u > R(0)) {
             const float rbar = 0.5f * ((float)rhoi + rhoj);
             const float vsig = rsqrt_(pair_div(fabsf((float)v.P[k] - (float)v.P[j]), rbar));
             dut += pair_div((float)alpha_u * mj * vsig * ((float)v.u[k] - (float)v.u[j]) * dW, rbar);
         }
-        kzu.add(f2(stz * mj - gz * mm, dut));
+        if constexpr (NG > 1) {
+            mine[5] = make_float4(axy.x, axy.y, 0.0f, 0.0f);
+            mine[6] = make_float4(stz * mj - gz * mm, dut, 0.0f, 0.0f);
+        } else {
+            kzu.add(f2(stz * mj - gz * mm, dut));
+        }
     };
     const float hs_pad = 2.0f * m;
     auto body = [&](int32_t j) {
@@ -2092,6 +2258,60 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
             traverse<R, LV>(v, I, pi, ci, pi.w + I.hmax_f + 2.0f * I.margin + 1e-6f * pi.w,
                      [&](int32_t j, float, float, float) { body(j); });
         }
+    } else if constexpr (NG > 1) {
+        const unsigned full = 0xffffffffu;
+        const bool use_list = live && !I.slack_flag && v.nbr_cnt[k] <= v.cap && v.xcnt[k] <= kExtraCap;
+        const int cnt = use_list ? v.nbr_cnt[k] : 0, all = cnt + (use_list ? v.xcnt[k] : 0);
+        const int32_t* nb = v.nbr + 4 * k;
+        auto entry = [&](int t) -> int32_t {
+            return t < cnt ? nb[nbr_slot(t, v.ls)] : (t < all ? v.xnbr[(int64_t)(t - cnt) * v.ls + k] : (int32_t)k);
+        };
+        float2 row = f2(0.0f);  // this lane's pair of the sums: rows of L (lanes 0 .. 4)
+        Kahan2 mom;             // ... momentum and energy (lanes 5, 6)
+        mom.init();
+        auto add_terms = [&](int n) {  // the group's first n entries, in order
+            if (g < 5) {
+                if (strength)
+                    for (int i = 0; i < n; i++) {
+                        const float4 q = group[i * kTerms + g];
+                        row = fma2(f2(q.x, q.y), f2(q.z, q.w), row);
+                    }
+            } else if (g < 7) {
+                for (int i = 0; i < n; i++) {
+                    const float4 q = group[i * kTerms + g];
+                    mom.add(f2(q.x, q.y));
+                }
+            }
+        };
+        const int most = __reduce_max_sync(full, all);
+        int32_t j = entry(g);
+        for (int t = 0; t < most; t += NG) {
+            const int32_t jn = entry(t + NG + g);  // the next entries' indices while these are evaluated
+            body(j);
+            __syncwarp();
+            add_terms(max(0, min(NG, all - t)));
+            __syncwarp();
+            j = jn;
+        }
+        if (live && !use_list) {  // the cells' particles one by one, the group in step
+            const unsigned gm = 0xffu << (threadIdx.x & 24);
+            traverse<R, LV>(v, I, pi, ci, pi.w + I.hmax_f + 2.0f * I.margin + 1e-6f * pi.w,
+                     [&](int32_t jj, float, float, float) {
+                         if (g == 0) body(jj);
+                         __syncwarp(gm);
+                         add_terms(1);
+                         __syncwarp(gm);
+                     });
+        }
+        __syncwarp();
+        auto of = [&](float2 x, int r) {
+            return f2(__shfl_sync(full, x.x, r, NG), __shfl_sync(full, x.y, r, NG));
+        };
+        Lp0 = of(row, 0); Lp1 = of(row, 1); Lp2 = of(row, 2); Lpz = of(row, 3);
+        Lp22 = of(row, 4).x;
+        kxy.s = of(mom.s, 5);
+        kzu.s = of(mom.s, 6);
+        if (!live || g != 0) return;
     } else if (!I.slack_flag && v.nbr_cnt[k] <= v.cap && v.xcnt[k] <= kExtraCap) {
         const int cnt = v.nbr_cnt[k];
         walk_list(v.nbr, v.ls, k, cnt, body);
@@ -2106,6 +2326,11 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
         L00 = Lp0.x; L01 = Lp0.y; L10 = Lp1.x; L11 = Lp1.y; L20 = Lp2.x; L21 = Lp2.y;
         L02 = Lpz.x; L12 = Lpz.y; L22 = Lp22;
         ax.s = kxy.s.x; ay.s = kxy.s.y; az.s = kzu.s.x; du.s = kzu.s.y;
+        // The rates below come out of the two forms of the sums (one lane, eight
+        // lanes) bit for bit alike: opaque scalars here, and the fused products
+        // written out where the compiler's choice between them varied.
+        asm volatile("" : "+f"(L00), "+f"(L01), "+f"(L02), "+f"(L10), "+f"(L11), "+f"(L12), "+f"(L20), "+f"(L21),
+                     "+f"(L22));
     }
     if constexpr (sizeof(R) == 8) {
         const double c = K<double>::inv_pi;
@@ -2120,20 +2345,21 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
         const R Rxy = R(0.5) * (L01 - L10), Rxz = R(0.5) * (L02 - L20), Ryz = R(0.5) * (L12 - L21);
         const R tr = rdiv(exx + eyy + ezz, R(3));
         // Jaumann J = R S - S R with R = [[0,Rxy,Rxz],[-Rxy,0,Ryz],[-Rxz,-Ryz,0]]
-        const R J00 = R(2) * (Rxy * sxy + Rxz * sxz);
-        const R J11 = R(2) * (-Rxy * sxy + Ryz * syz);
-        const R J22 = R(2) * (-Rxz * sxz - Ryz * syz);
-        const R J01 = Rxy * syy + Rxz * syz - sxx * Rxy + sxz * Ryz;
-        const R J02 = Rxy * syz + Rxz * szz - sxx * Rxz - sxy * Ryz;
-        const R J12 = -Rxy * sxz + Ryz * szz - sxy * Rxz - syy * Ryz;
+        const R bxy = rmul(Rxy, sxy), byz = rmul(Ryz, syz);
+        const R h00 = rfma(Rxz, sxz, bxy), h11 = byz - bxy;  // J00 / 2, J11 / 2
+        const R h22 = rfma(-Rxz, sxz, -byz);  // J22 / 2
+        const R J01 = rfma(sxz, Ryz, rfma(-sxx, Rxy, rfma(Rxz, syz, rmul(Rxy, syy))));
+        const R J02 = rfma(-sxy, Ryz, rfma(-sxx, Rxz, rfma(Rxz, szz, rmul(Rxy, syz))));
+        const R J12 = rfma(-syy, Ryz, rfma(-sxy, Rxz, rfma(Ryz, szz, -rmul(Rxy, sxz))));
         const R twoG = R(2) * G;
-        v.dS_new[0][k] = twoG * (exx - tr) + J00;
-        v.dS_new[1][k] = twoG * (eyy - tr) + J11;
-        v.dS_new[2][k] = twoG * (ezz - tr) + J22;
-        v.dS_new[3][k] = twoG * exy + J01;
-        v.dS_new[4][k] = twoG * exz + J02;
-        v.dS_new[5][k] = twoG * eyz + J12;
-        epsw = rdiv(sxx * exx + syy * eyy + szz * ezz + R(2) * (sxy * exy + sxz * exz + syz * eyz), rhoi);
+        v.dS_new[0][k] = rfma(twoG, exx - tr, R(2) * h00);
+        v.dS_new[1][k] = rfma(twoG, eyy - tr, R(2) * h11);
+        v.dS_new[2][k] = rfma(R(2), h22, rmul(twoG, ezz - tr));
+        v.dS_new[3][k] = rfma(twoG, exy, J01);
+        v.dS_new[4][k] = rfma(twoG, exz, J02);
+        v.dS_new[5][k] = rfma(twoG, eyz, J12);
+        const R dn = rfma(szz, ezz, rfma(syy, eyy, rmul(sxx, exx))), ds = rfma(syz, eyz, rfma(sxz, exz, rmul(sxy, exy)));
+        epsw = rdiv(rfma(R(2), ds, dn), rhoi);
     } else {
 #pragma unroll
         for (int c = 0; c < 6; c++) v.dS_new[c][k] = R(0);
