@@ -77,6 +77,7 @@ struct Visc {
     double *rr, *zz, *pp[2], *qq;
     double* part;  // per-block partial sums, two sets of [3][nblk] used in turn
     int nblk;
+    bool cluster;  // the blocks run as one thread-block cluster
 };
 
 // Polls of the barrier generation before a block gives up (~0.1-1 s).
@@ -115,6 +116,18 @@ static __device__ bool grid_barrier(Ctl* ctl, unsigned nblk) {
     return ok != 0;
 }
 
+// All the launch's blocks: in one thread-block cluster, the hardware's cluster
+// barrier (release / acquire, no wait loop); otherwise the grid-wide one.
+template <bool CLUSTER>
+static __device__ __forceinline__ bool all_blocks(Ctl* ctl, unsigned nblk) {
+    if constexpr (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    } else {
+        return grid_barrier(ctl, nblk);
+    }
+}
+
 // The block's sums of K per-thread values into part[k * nblk + block].
 template <int K>
 static __device__ void block_partials(const double (&v)[K], double* part, unsigned nblk) {
@@ -145,9 +158,16 @@ static __device__ double grid_total(const double* part, int k, unsigned nblk) {
 }
 
 static __device__ __forceinline__ double harmonic(double a, double b) {
-    return (a > 0 && b > 0) ? 2.0 * a * b / (a + b) : 0.0;
+    return (gt0(a) && gt0(b)) ? dv(2.0 * a * b, a + b) : 0.0;
 }
 
+// CLUSTER: a grid of at most kViscCluster blocks runs as one thread-block
+// cluster.  A phase between barriers is a microsecond or two of work there, and
+// the grid-wide barrier through L2 took about as long (60 x 44 cells, 11 blocks,
+// 20 iterations a step: 403 -> 333 us a mixed step).  The same blocks, cells and
+// order of sums either way.
+constexpr int kViscCluster = 16;
+template <bool CLUSTER>
 static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, Visc w, Ctl* ctl) {
     if (!ctl->active) return;
     const double dt = ctl->dt, dx = p.dx, rmin = dmax2(p.rho_cfl, 1e-12);
@@ -164,9 +184,10 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         return s;
     };
     auto ijk = [&](int64_t c, int& i, int& j, int& k) {
-        i = (int)(c / sx);
-        j = (int)((c / nz) % ny);
-        k = (int)(c % nz);
+        const uint32_t line = (uint32_t)c / (uint32_t)nz;
+        k = (int)((uint32_t)c - line * (uint32_t)nz);
+        i = (int)(line / (uint32_t)ny);
+        j = (int)(line - (uint32_t)i * (uint32_t)ny);
     };
     auto cell_volume = [&](int i) {  // hydro_cpu.cpp:309
         const double rc = (i + 0.5) * dx, wV = ax ? rc : dx;
@@ -183,7 +204,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         }
         double* part = sums();
         block_partials<1>(v, part, nb);
-        if (!grid_barrier(ctl, nb)) return;
+        if (!all_blocks<CLUSTER>(ctl, nb)) return;
         if (grid_total(part, 0, nb) == 0) return;  // nothing fluidized: no change
     }
     // face coefficients dt A_f eta_f / dx and the curvature diagonal
@@ -194,9 +215,9 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         w.cfx[c] = i < nx - 1 ? dt * (ax ? (i + 1) * dx : dx) * harmonic(e, __ldcg(w.eta + c + sx)) : 0.0;
         w.cfy[c] = (ny > 1 && j < ny - 1) ? dt * dx * harmonic(e, __ldcg(w.eta + c + sy)) : 0.0;
         w.cfz[c] = k < nz - 1 ? dt * wV * harmonic(e, __ldcg(w.eta + c + 1)) : 0.0;
-        w.dax[c] = ax ? dt * e * Vc / (rc * rc) : 0.0;
+        w.dax[c] = ax ? dv(dt * e * Vc, rc * rc) : 0.0;
     }
-    if (!grid_barrier(ctl, nb)) return;
+    if (!all_blocks<CLUSTER>(ctl, nb)) return;
     // diagonal: the cell's mass and every face coefficient it touches, added
     // in the order of the reference's scatter loop (hydro_cpu.cpp:315-319)
     for (int64_t c = c0; c < n; c += stride) {
@@ -211,7 +232,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         if (k < nz - 1) s += __ldcg(w.cfz + c);
         w.dsum[c] = s;
     }
-    if (!grid_barrier(ctl, nb)) return;
+    if (!all_blocks<CLUSTER>(ctl, nb)) return;
 
     // y = A x at cell c (hydro_cpu.cpp:321-331), x given per cell by xv
     auto amul = [&](int64_t c, int i, int j, int k, bool wd, auto xv) {
@@ -236,13 +257,13 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         {  // initial guess: the current velocity; right-hand side Vc (rho v)
             double v[1] = {0};
             for (int64_t c = c0; c < n; c += stride) {
-                const double b = cell_volume((int)(c / sx)) * mom[c];
-                x[c] = mom[c] / r[c];
+                const double b = cell_volume((int)((uint32_t)c / (uint32_t)sx)) * mom[c];
+                x[c] = dv(mom[c], r[c]);
                 v[0] += b * b;
             }
             double* part = sums();
             block_partials<1>(v, part, nb);
-            if (!grid_barrier(ctl, nb)) return;
+            if (!all_blocks<CLUSTER>(ctl, nb)) return;
             bn = grid_total(part, 0, nb);
         }
         if (bn <= 0) {
@@ -256,7 +277,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
                 ijk(c, i, j, k);
                 const double q = amul(c, i, j, k, wd, [&](int64_t cc) { return __ldcg(x + cc); });
                 const double rv = cell_volume(i) * mom[c] - q;
-                const double zv = rv / diag(c, wd);
+                const double zv = dv(rv, diag(c, wd));
                 w.rr[c] = rv;
                 w.zz[c] = zv;
                 w.pp[0][c] = zv;
@@ -265,7 +286,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
             }
             double* part = sums();
             block_partials<2>(v, part, nb);
-            if (!grid_barrier(ctl, nb)) return;
+            if (!all_blocks<CLUSTER>(ctl, nb)) return;
             rn = grid_total(part, 0, nb);
             rz = grid_total(part, 1, nb);
         }
@@ -294,11 +315,11 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
                 if (!first) cur ^= 1;
                 double* part = sums();
                 block_partials<1>(v, part, nb);
-                if (!grid_barrier(ctl, nb)) return;
+                if (!all_blocks<CLUSTER>(ctl, nb)) return;
                 pq = grid_total(part, 0, nb);
             }
             if (pq <= 0) break;
-            const double al = rz / pq;
+            const double al = dv(rz, pq);
             double rz2;
             {  // x += alpha p, r -= alpha q, z = r / diag
                 const double* pc = cur ? w.pp[1] : w.pp[0];
@@ -307,24 +328,24 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
                     x[c] += al * pc[c];
                     const double rv = w.rr[c] - al * w.qq[c];
                     w.rr[c] = rv;
-                    const double zv = rv / diag(c, wd);
+                    const double zv = dv(rv, diag(c, wd));
                     w.zz[c] = zv;
                     v[0] += rv * rv;
                     v[1] += rv * zv;
                 }
                 double* part = sums();
                 block_partials<2>(v, part, nb);
-                if (!grid_barrier(ctl, nb)) return;
+                if (!all_blocks<CLUSTER>(ctl, nb)) return;
                 rn = grid_total(part, 0, nb);
                 rz2 = grid_total(part, 1, nb);
             }
             if (blockIdx.x == 0 && threadIdx.x == 0) ctl->visc_iters++;
             if (rn <= tol2) break;
-            be = rz2 / rz;
+            be = dv(rz2, rz);
             rz = rz2;
         }
     }
-    if (!grid_barrier(ctl, nb)) return;  // every cell's new velocity in place
+    if (!all_blocks<CLUSTER>(ctl, nb)) return;  // every cell's new velocity in place
 
     // heating: the kinetic energy removed, spread over the cells in
     // proportion to the dissipation of their faces (hydro_cpu.cpp:355-376)
@@ -342,7 +363,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
             ijk(c, i, j, k);
             const double rho = r[c], mu = g.q[F_MU][c], mv = g.q[F_MV][c], mw = g.q[F_MW][c];
             const double uc = __ldcg(u1 + c), vc = __ldcg(v1 + c), wc = __ldcg(w1 + c), Vc = cell_volume(i);
-            const double keo = 0.5 * (mu * mu + mv * mv + mw * mw) / rho;
+            const double keo = dv(0.5 * (mu * mu + mv * mv + mw * mw), rho);
             const double ken = 0.5 * rho * (uc * uc + vc * vc + wc * wc);
             v[0] += keo * Vc;
             v[1] += ken * Vc;
@@ -354,7 +375,7 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         }
         double* part = sums();
         block_partials<3>(v, part, nb);
-        if (!grid_barrier(ctl, nb)) return;
+        if (!all_blocks<CLUSTER>(ctl, nb)) return;
         const double totold = grid_total(part, 0, nb), totnew = grid_total(part, 1, nb),
                      htot = grid_total(part, 2, nb);
         const double loss = totold - totnew;
@@ -377,14 +398,14 @@ static __global__ void __launch_bounds__(256, 3) k_implicit_visc(P p, Fields g, 
         double& mu = g.q[F_MU][c];
         double& mv = g.q[F_MV][c];
         double& mw = g.q[F_MW][c];
-        const double keo = 0.5 * (mu * mu + mv * mv + mw * mw) / rho;
+        const double keo = dv(0.5 * (mu * mu + mv * mv + mw * mw), rho);
         mu = rho * uc;
         mv = rho * vc;
         mw = rho * wc;
-        const double ken = 0.5 * (mu * mu + mv * mv + mw * mw) / rho;
-        double q = sc * hr / cell_volume(i);
+        const double ken = dv(0.5 * (mu * mu + mv * mv + mw * mw), rho);
+        double q = dv(sc * hr, cell_volume(i));
         if (p.af_reg && q > 0) {  // C_REG of the dissipation regenerates vibrations
-            g.q[F_VIB][c] = sqrt(g.q[F_VIB][c] * g.q[F_VIB][c] + 2.0 * p.c_reg * q / rho);
+            g.q[F_VIB][c] = root(g.q[F_VIB][c] * g.q[F_VIB][c] + dv(2.0 * p.c_reg * q, rho));
             q *= (1.0 - p.c_reg);
         }
         g.q[F_E][c] += (ken - keo) + q;
@@ -477,18 +498,51 @@ struct Grid {
         EU_CUDA(cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device));
         if (!dev_coop) throw SphError(SPH_ERR_CUDA, "the implicit viscosity needs cooperative launches");
         EU_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-        EU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_implicit_visc, 256, 0));
+        EU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_implicit_visc<false>, 256, 0));
         if (per_sm < 1) throw SphError(SPH_ERR_CUDA, "implicit viscosity kernel does not fit on an SM");
         const int64_t want = std::max<int64_t>(1, (p.n + 255) / 256);
         vw.nblk = (int)std::min<int64_t>(want, (int64_t)per_sm * nsm);
+        vw.cluster = vw.nblk == want && want <= kViscCluster && visc_cluster_fits(vw.nblk);
         for (double** a : {&vw.eta, &vw.cfx, &vw.cfy, &vw.cfz, &vw.dax, &vw.dsum, &vw.x[0], &vw.x[1], &vw.x[2],
                            &vw.rr, &vw.zz, &vw.pp[0], &vw.pp[1], &vw.qq})
             *a = alloc(p.n);
         vw.part = alloc(6 * (int64_t)vw.nblk);
     }
 
+    // The launch of one cluster of nblk blocks (attr: the caller's storage).
+    cudaLaunchConfig_t visc_cluster_config(int nblk, cudaLaunchAttribute* attr) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)nblk);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        attr->id = cudaLaunchAttributeClusterDimension;
+        attr->val.clusterDim.x = (unsigned)nblk;
+        attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cfg;
+    }
+    // Can a cluster of nblk blocks be resident (above 8 needs the opt-in)?
+    bool visc_cluster_fits(int nblk) {
+        cudaLaunchAttribute attr{};
+        const cudaLaunchConfig_t cfg = visc_cluster_config(nblk, &attr);
+        int fit = 0;
+        const bool ok = cudaFuncSetAttribute(k_implicit_visc<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                            cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&fit, k_implicit_visc<true>, &cfg) == cudaSuccess && fit >= 1;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
+
     void enqueue_visc() {
         ensure_visc();
+        if (vw.cluster) {
+            cudaLaunchAttribute attr{};
+            const cudaLaunchConfig_t cfg = visc_cluster_config(vw.nblk, &attr);
+            EU_CUDA(cudaLaunchKernelEx(&cfg, k_implicit_visc<true>, p, g, vw, ctl));
+            launches++;
+            return;
+        }
         static_assert(offsetof(Ctl, visc_err) == offsetof(Ctl, bar_count) + 4, "barrier fields are adjacent");
         EU_CUDA(cudaMemsetAsync(&ctl->bar_count, 0, 8, st));  // barrier count and error flag
         P pv = p;
@@ -496,7 +550,7 @@ struct Grid {
         Visc wv = vw;
         Ctl* cv = ctl;
         void* args[] = {&pv, &gv, &wv, &cv};
-        EU_CUDA(cudaLaunchCooperativeKernel((const void*)k_implicit_visc, dim3((unsigned)vw.nblk), dim3(256), args, 0, st));
+        EU_CUDA(cudaLaunchCooperativeKernel((const void*)k_implicit_visc<false>, dim3((unsigned)vw.nblk), dim3(256), args, 0, st));
         launches++;
     }
 
@@ -1047,8 +1101,10 @@ int eu_run(eu_grid* h, double cfl, double t_end, int64_t max_steps, int64_t* ste
         g->launches++;
         const deu::Ctl c0 = g->read_ctl();
         // The implicit viscosity's cooperative launch is issued directly, not
-        // from a graph: steps with it are enqueued one by one.
-        const bool direct = g->visc_on();
+        // from a graph: steps with it are enqueued one by one (as a cluster it is
+        // a kernel like the others).
+        if (g->visc_on()) g->ensure_visc();
+        const bool direct = g->visc_on() && !g->vw.cluster;
         if (!direct && !g->graph_valid) {  // one driver step, captured once per settings
             if (g->graph) cudaGraphExecDestroy(g->graph);
             g->graph = nullptr;
