@@ -1617,11 +1617,20 @@ private:
     // force 69 / 23; 22,040: 94 / 52, 47 / 31, 66 / 50; 39,464: 98 / 86, 45 / 42,
     // 67 / 74; 64,280: 109 / 95, 49 / 61, 78 / 111; 85,544: 117 / 121 (list).
     static constexpr int64_t kFewParticles = 32768, kFewForLists = 65536;
+    // The FP64 form's pair passes take four lanes to a particle at every count:
+    // its results may not depend on which impacts are resident, and the lanes'
+    // partial sums do depend on their number.  One thread / 2 / 4 / 8 lanes, us:
+    // force of 6k particles 414 / 212 / 142 / 109, 20k 495 / 373 / 360 / 306,
+    // 57k 793 / 757 / 741 / 753, 131k 1683 / 1613 / 1605 / 1690; density 215 /
+    // 111 / 64 / 58, 215 / 180 / 172 / 153, 378 / 358 / 283 / 319, 672 / 620 /
+    // 615 / 705.  Eight lanes lose to the last, partly filled trip of a list.
+    static constexpr int kLanes64 = 4;
     bool few_particles() const { return sizeof(R) == 4 && N_ <= kFewParticles && !levels_active_ && !any_periodic(); }
     void launch_force() {
         if (N_ <= 0) return;
         prof_begin();
-        const unsigned grid = (unsigned)((N_ + 127) / 128);
+        constexpr int L = sizeof(R) == 8 ? kLanes64 : 1;
+        const unsigned grid = (unsigned)((L * N_ + 127) / 128);
         bool done = false;
         if (sizeof(R) == 4 && !levels_active_) {
             done = true;
@@ -1635,19 +1644,19 @@ private:
             }
         }
         if (levels_active_) {  // graded impacts resident: the level-aware pass (never staged)
-            k_force<R, 0, 0, false, true><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
-            launched((const void*)k_force<R, 0, 0, false, true>);
+            k_force<R, 0, 0, false, true, true, L><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
+            launched((const void*)k_force<R, 0, 0, false, true, true, L>);
         } else if (!done && any_periodic()) {
-            k_force<R, 0, 0, false, false, true><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
-            launched((const void*)k_force<R, 0, 0, false, false, true>);
+            k_force<R, 0, 0, false, false, true, L><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
+            launched((const void*)k_force<R, 0, 0, false, false, true, L>);
         } else if (!done && few_particles()) {
             if constexpr (sizeof(R) == 4) {
                 k_force<R, 0, 0, false, false, false, 8><<<(unsigned)((8 * N_ + 127) / 128), 128, 0, st_>>>(view(), wait_err_d_);
                 launched((const void*)k_force<R, 0, 0, false, false, false, 8>);
             }
         } else if (!done) {  // no resident impact is periodic: pair loop without minimum image
-            k_force<R, 0, 0, false, false, false><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
-            launched((const void*)k_force<R, 0, 0, false, false, false>);
+            k_force<R, 0, 0, false, false, false, L><<<grid, 128, 0, st_>>>(view(), wait_err_d_);
+            launched((const void*)k_force<R, 0, 0, false, false, false, L>);
         }
         prof_end();
         launches_++;
@@ -2522,12 +2531,13 @@ public:
             if (round > 0) launch_n_raw(k_ref_bins<R>, N_, view(), 0);
             cls(KC_DENSITY);
             if (iters > 0) {  // also reduces the new max h
-                if (levels_active_) launch_n_raw(k_density<R, true>, N_, view(), iters);
-                else if (any_periodic()) launch_n_raw(k_density<R, false, true>, N_, view(), iters);
+                constexpr int L = sizeof(R) == 8 ? kLanes64 : 1;
+                if (levels_active_) launch_n_raw(k_density<R, true, true, L>, L * N_, view(), iters);
+                else if (any_periodic()) launch_n_raw(k_density<R, false, true, L>, L * N_, view(), iters);
                 else if (few_particles()) {
                     if constexpr (sizeof(R) == 4) launch_n_raw(k_density<R, false, false, 8>, 8 * N_, view(), iters);
                 }
-                else launch_n_raw(k_density<R, false, false>, N_, view(), iters);
+                else launch_n_raw(k_density<R, false, false, L>, L * N_, view(), iters);
             }
             else hmax_pass(1);
             cls(KC_GRID);

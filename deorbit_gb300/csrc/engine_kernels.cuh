@@ -1697,6 +1697,14 @@ struct Kahan2 {
     }
 };
 
+// Sum over the G lanes of a group, the same in each of them.
+template <int G>
+__device__ __forceinline__ double group_sum(double x) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
 // Does particle k's superset list still cover it (count within capacity and h
 // within the slack, with an allowance for the FP32 distance)?
 template <class R>
@@ -1713,7 +1721,7 @@ __device__ __forceinline__ bool list_covers(const View<R>& v, const ImpactD& I, 
 // once; every lane then adds them in list order, so the sums are the same.
 template <class R, bool LV = false, bool PER = true, int G = 1>
 static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(View<R> v, int iters) {
-    static_assert(G == 1 || (sizeof(R) == 4 && !LV && !PER), "lane groups: mixed form, one grid, no periodic axis");
+    static_assert(G == 1 || sizeof(R) == 8 || (!LV && !PER), "mixed form's lane groups: one grid, no periodic axis");
     int64_t k = gtid() / G;
     bool act = k < v.n;
     if (G == 1 && !act) return;
@@ -1721,14 +1729,36 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
     ImpactD& I = v.imps[v.imp[k]];
     act = act && I.mask && I.active;
     if (G == 1 && !act) return;
+    constexpr bool kGroup64 = G > 1 && sizeof(R) == 8;
+    if (kGroup64) {
+        if (!__syncthreads_or(act)) return;
+    } else if (G > 1 && !__any_sync(0xffffffffu, act)) {
+        return;
+    }
     [[maybe_unused]] const int g = threadIdx.x & (G - 1);
     R hi = v.hh[k];
     const float4 pi = v.pf[k];
     const uint32_t ci = v.cpk[k];
     const unsigned long long bi = v.refbin[k];
     const float m = sizeof(R) == 8 ? I.margin : 0.0f;
-    const R mass_k = v.mass[k];
-    const R h0 = I.use_h0 ? v.h0[k] : (R)I.h_init;
+    // FP64 groups: one thread a particle finishes the sums, in whole warps (a
+    // quarter of every warp would hold the FP64 pipe as long as a full one:
+    // 131,072 particles 640 -> 615 us, 57,472: 294 -> 283)
+    constexpr int kOwn = 256 / G;
+    __shared__ double fin[kGroup64 ? 3 : 1][kGroup64 ? kOwn : 1];
+    [[maybe_unused]] const int own = (int)(threadIdx.x + 256 - 64 * (blockIdx.x & 3)) & 255;
+    const int64_t kf = kGroup64 ? (int64_t)blockIdx.x * kOwn + own : k;
+    bool finishes = false;
+    if constexpr (kGroup64) {
+        finishes = own < kOwn && kf < v.n;
+        if (finishes) {
+            const ImpactD& If = v.imps[v.imp[kf]];
+            finishes = If.mask && If.active;
+        }
+    }
+    ImpactD& If = kGroup64 && finishes ? v.imps[v.imp[kf]] : I;
+    const R mass_k = v.mass[finishes ? kf : k];
+    const R h0 = If.use_h0 ? v.h0[finishes ? kf : k] : (R)If.h_init;
     double xi = 0.0, yi = 0.0, zi = 0.0;
     if constexpr (sizeof(R) == 8) { xi = v.x[k]; yi = v.y[k]; zi = v.z[k]; }
     R rho = R(1e-30), rho_lo = R(0);
@@ -1755,7 +1785,8 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
                 // FP32 distance: outside and inside are clear except within the
                 // margin of 2 h, where the reference's exact test decides
                 // (131,072 particles, both iterations: 1.51 -> 0.68 ms with it,
-                // the integer root and the common factors out of the sum)
+                // the integer root and the common factors out of the sum;
+                // 0.61 with four lanes to a particle)
                 float fx, fy, fz;
                 sep_f32<PER>(I, pi, ci, v.pf[j], v.cpk[j], fx, fy, fz);
                 const float f2 = fx * fx + fy * fy + fz * fz;
@@ -1773,7 +1804,26 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
                 sum.add((R)w_mixed(j, v.pf[j], v.pk[j]));
             }
         };
-        if constexpr (G > 1) {
+        if constexpr (G > 1 && sizeof(R) == 8) {
+            if (act) {
+                if (list_covers(v, I, k, (float)hi)) {
+                    const int cnt = v.nbr_cnt[k];
+                    const int32_t* nb = v.nbr + 4 * k;
+                    int32_t j = g < cnt ? nb[nbr_slot(g, v.ls)] : 0;
+                    for (int t = g; t < cnt; t += G) {
+                        const int32_t jn = t + G < cnt ? nb[nbr_slot(t + G, v.ls)] : 0;
+                        body(j);
+                        j = jn;
+                    }
+                } else {
+                    const float hf = (float)hi;
+                    int at = 0;
+                    traverse<R, LV>(v, I, pi, ci, 2.0f * hf * 1.0001f + 2.0f * I.margin + 1e-6f * hf,
+                             [&](int32_t j, float, float, float) { if ((at++ & (G - 1)) == g) body(j); });
+                }
+            }
+            sum.s = group_sum<G>(sum.s);
+        } else if constexpr (G > 1) {
             const unsigned full = 0xffffffffu;
             const bool covers = act && list_covers(v, I, k, (float)hi);
             const int cnt = covers ? v.nbr_cnt[k] : 0;
@@ -1821,21 +1871,39 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_density(
             traverse<R, LV>(v, I, pi, ci, 2.0f * hf * 1.0001f + 2.0f * I.margin + 1e-6f * hf,
                      [&](int32_t j, float, float, float) { body(j); });
         }
-        if constexpr (sizeof(R) == 8) sum.s *= 0.25 * K<double>::inv_pi * ihi * ihi * ihi;
-        rho = rmax(sum.value(), R(1e-30));
-        rho_lo = rho > R(1e-30) ? sum.low() : R(0);
-        hi = rmin(R(2) * h0, rmax(R(0.5) * h0, (R)I.eta * rcbrt(rdiv(mass_k, rho))));
+        if constexpr (kGroup64) {
+            if (g == 0) { fin[0][threadIdx.x / G] = sum.s; fin[1][threadIdx.x / G] = ihi; }
+            __syncthreads();
+            if (finishes) {
+                const double ih = fin[1][own];
+                rho = rmax(fin[0][own] * (0.25 * K<double>::inv_pi * ih * ih * ih), 1e-30);
+                hi = rmin(2.0 * h0, rmax(0.5 * h0, If.eta * rcbrt(rdiv(mass_k, rho))));
+                fin[2][own] = hi;
+            }
+            if (it + 1 < iters) {
+                __syncthreads();
+                hi = fin[2][threadIdx.x / G];
+            }
+        } else {
+            if constexpr (sizeof(R) == 8) sum.s *= 0.25 * K<double>::inv_pi * ihi * ihi * ihi;
+            rho = rmax(sum.value(), R(1e-30));
+            rho_lo = rho > R(1e-30) ? sum.low() : R(0);
+            hi = rmin(R(2) * h0, rmax(R(0.5) * h0, (R)I.eta * rcbrt(rdiv(mass_k, rho))));
+        }
     }
-    if (G > 1 && !act) return;
-    impact_atomic_max(&I.hm_bits, (double)hi);  // the round's new max h
-    if (G > 1 && g != 0) return;
+    if (kGroup64) {
+        if (!finishes) return;
+        k = kf;
+    } else if (G > 1 && !act) return;
+    impact_atomic_max(&If.hm_bits, (double)hi);  // the round's new max h
+    if (!kGroup64 && G > 1 && g != 0) return;
     v.rho[k] = rho;
     v.rho_lo[k] = rho_lo;
     v.hh[k] = hi;
     v.pf[k].w = (float)hi;
     v.lf[k].w = (float)hi;
-    if (!((float)hi <= v.hlist[k] * (1.0f + I.slack) * 0.99999f)) {
-        atomicOr(&I.slack_flag, 1);
+    if (!((float)hi <= v.hlist[k] * (1.0f + If.slack) * 0.99999f)) {
+        atomicOr(&If.slack_flag, 1);
         atomicOr(&v.flags[2], 1);
     }
 }
@@ -1961,10 +2029,11 @@ template <class R, int SE = 0, int SS = 0, bool ASYNC = false, bool LV = false, 
 static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(View<R> v, int32_t* wait_err) {
     using Acc = AccT<R>;
     constexpr bool kStaged = SS > 0 && sizeof(R) == 4;
-    static_assert(NG == 1 || (NG == 8 && sizeof(R) == 4 && !kStaged && !LV && !PER),
-                  "lane groups: mixed form, one grid, no periodic axis");
+    constexpr bool kGroup64 = NG > 1 && sizeof(R) == 8;
+    static_assert(NG == 1 || kGroup64 || (NG == 8 && !kStaged && !LV && !PER),
+                  "mixed form's lane groups: one grid, no periodic axis");
     constexpr int kTerms = 7;  // per entry: four packed rows of L, L22, (ax, ay), (az, du)
-    __shared__ float4 terms[NG > 1 ? 128 * kTerms : 1];
+    __shared__ float4 terms[NG > 1 && !kGroup64 ? 128 * kTerms : 1];
     [[maybe_unused]] const int g = threadIdx.x & (NG - 1);
     [[maybe_unused]] float4* const mine = terms + (NG > 1 ? threadIdx.x * kTerms : 0);
     [[maybe_unused]] const float4* const group = terms + (NG > 1 ? (threadIdx.x - g) * kTerms : 0);
@@ -1979,18 +2048,19 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
         if (!I.mask) return;
     }
     live = live && I.mask;
-    const R G = v.mats[v.mat[k]].G;
-    const bool strength = G > R(0);
+    R G = v.mats[v.mat[k]].G;
+    bool strength = G > R(0);
     const R alpha = (R)I.alpha, beta = (R)I.beta, eps = (R)I.eps, eps_as = (R)I.eps_as;
     const R alpha_u = (R)I.alpha_u, half_alpha = R(0.5) * alpha;
     const R inv_poly = sizeof(R) == 4 ? (R)I.inv_poly_eta_f : (R)I.inv_poly_eta;
-    const R hi = v.hh[k], rhoi = v.rho[k], csi = v.csig[k], Pi_over = v.pfr2[k];
+    R rhoi = v.rho[k];
+    const R hi = v.hh[k], csi = v.csig[k], Pi_over = v.pfr2[k];
     const R dsri = v.dsr2[k], Rai = v.Rart[k];
     const double vxi = v.vx[k], vyi = v.vy[k], vzi = v.vz[k];
     float4 vhi = make_float4(0, 0, 0, 0), vli = vhi;
     if (sizeof(R) == 4) { vhi = v.fr[6 * k + 1]; vli = v.fr[6 * k + 2]; }
-    const R sxx = v.S[0][k], syy = v.S[1][k], szz = v.S[2][k];
-    const R sxy = v.S[3][k], sxz = v.S[4][k], syz = v.S[5][k];
+    R sxx = v.S[0][k], syy = v.S[1][k], szz = v.S[2][k];
+    R sxy = v.S[3][k], sxz = v.S[4][k], syz = v.S[5][k];
     R L00 = 0, L01 = 0, L02 = 0, L10 = 0, L11 = 0, L12 = 0, L20 = 0, L21 = 0, L22 = 0;
     Acc ax, ay, az, du;
     ax.init(); ay.init(); az.init(); du.init();
@@ -2102,7 +2172,7 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
             // work, grad W stays factored as wg d, and the stress and pressure
             // terms act as one tensor.  131,072 particles with strength: 200 ->
             // 108 pipe slots a pair, 3.48 -> 1.88 ms (three resident blocks; 2.05
-            // at two, 1.98 at four).
+            // at two, 1.98 at four); 1.60 with four lanes to a particle.
             if (j == (int32_t)k) return;
             const float4 pjf = v.pf[j];
             float fx, fy, fz;  // FP32 distance: the exact test only within its margin of h_i + h_j
@@ -2258,6 +2328,47 @@ static __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_force(Vi
             traverse<R, LV>(v, I, pi, ci, pi.w + I.hmax_f + 2.0f * I.margin + 1e-6f * pi.w,
                      [&](int32_t j, float, float, float) { body(j); });
         }
+    } else if constexpr (kGroup64) {
+        if (live) {
+            if (!I.slack_flag && v.nbr_cnt[k] <= v.cap && v.xcnt[k] <= kExtraCap) {
+                const int cnt = v.nbr_cnt[k], all = cnt + v.xcnt[k];
+                const int32_t* nb = v.nbr + 4 * k;
+                auto entry = [&](int t) -> int32_t {
+                    return t < cnt ? nb[nbr_slot(t, v.ls)] : (t < all ? v.xnbr[(int64_t)(t - cnt) * v.ls + k] : (int32_t)k);
+                };
+                int32_t j = entry(g);
+                for (int t = g; t < all; t += NG) {
+                    const int32_t jn = entry(t + NG);
+                    body(j);
+                    j = jn;
+                }
+            } else {
+                int at = 0;
+                traverse<R, LV>(v, I, pi, ci, pi.w + I.hmax_f + 2.0f * I.margin + 1e-6f * pi.w,
+                         [&](int32_t j, float, float, float) { if ((at++ & (NG - 1)) == g) body(j); });
+            }
+        }
+        // One thread a particle finishes the rates, in whole warps (a quarter of
+        // every warp would hold the FP64 pipe as long as a full one); the warp
+        // moves with the block, its sub-partition with it.
+        __shared__ double sums[13][128 / NG];
+        double* const s13[] = {&L00, &L01, &L02, &L10, &L11, &L12, &L20, &L21, &L22, &ax.s, &ay.s, &az.s, &du.s};
+#pragma unroll
+        for (int c = 0; c < 13; c++) {
+            const double x = group_sum<NG>(*s13[c]);
+            if (g == 0) sums[c][threadIdx.x / NG] = x;
+        }
+        __syncthreads();
+        const int at = (int)(threadIdx.x + 128 - 32 * (blockIdx.x & 3)) & 127;
+        k = (int64_t)blockIdx.x * (128 / NG) + at;
+        if (at >= 128 / NG || k >= v.n || !v.imps[v.imp[k]].mask) return;
+#pragma unroll
+        for (int c = 0; c < 13; c++) *s13[c] = sums[c][at];
+        G = v.mats[v.mat[k]].G;
+        strength = G > R(0);
+        rhoi = v.rho[k];
+        sxx = v.S[0][k]; syy = v.S[1][k]; szz = v.S[2][k];
+        sxy = v.S[3][k]; sxz = v.S[4][k]; syz = v.S[5][k];
     } else if constexpr (NG > 1) {
         const unsigned full = 0xffffffffu;
         const bool use_list = live && !I.slack_flag && v.nbr_cnt[k] <= v.cap && v.xcnt[k] <= kExtraCap;
