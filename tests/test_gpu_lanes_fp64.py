@@ -51,3 +51,33 @@ def test_sizes_match_oracle(cuda_lib, oracle_lib, n, how):
     errs = field_errors(read_all(ctx, b, names), {k: orc.field(k) for k in names}, names)
     ctx.close()
     assert max(errs.values()) <= 1e-9, errs
+
+
+@pytest.mark.parametrize("strength", [False, True])
+def test_written_stress_matches_oracle(cuda_lib, oracle_lib, strength):
+    """An impact without stress leaves the stress terms out of its force pass; one particle's stress, written
+    between two steps, brings them back (and the written zeros take them out again)."""
+    from deorbit_gb300 import sph
+    sc = few(515)
+    if not strength:
+        sc.materials = [ic.granite(strength=False), ic.iron(strength=False)]
+    ctx = sph.Context(sph.FP64)
+    b = ic.to_context(ctx, sc)
+    orc = O.from_scenario(sc)
+    ctx.init()
+    orc.init()
+    names = [k for k in STATE + DERIV if strength or k not in ("dSxx", "dSyy", "dSzz", "dSxy", "dSxz", "dSyz")]
+    for stress in (None, 3.0e8, 0.0):
+        if stress is not None:
+            for k in ("Sxx", "Sxy"):
+                s = orc.field(k)
+                s[:] = 0.0
+                s[200] = stress
+                orc.set_field(k, s)
+                ctx.write(b, k, s)
+        dt = orc.timestep()
+        orc.step(dt)
+        ctx.step(dt)
+        errs = field_errors(read_all(ctx, b, names), {k: orc.field(k) for k in names}, names)
+        assert max(errs.values()) <= 1e-9, (stress, errs)
+    ctx.close()
