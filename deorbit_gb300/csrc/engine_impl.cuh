@@ -1610,13 +1610,14 @@ private:
             if (h.used && h.alive && (h.per[0] | h.per[1] | h.per[2])) return true;
         return false;
     }
-    // Runs of few particles take eight lanes to a particle in the list build and
-    // the mixed form's pair passes (same results): below these counts the
-    // thread-per-particle kernels leave SMs with too few warps to cover a pair's
-    // loads.  Thread / lanes, us: 5,864 particles list 98 / 46, density 47 / 18,
-    // force 69 / 23; 22,040: 94 / 52, 47 / 31, 66 / 50; 39,464: 98 / 86, 45 / 42,
-    // 67 / 74; 64,280: 109 / 95, 49 / 61, 78 / 111; 85,544: 117 / 121 (list).
-    static constexpr int64_t kFewParticles = 32768, kFewForLists = 65536;
+    // Runs of few particles take a warp to a particle in the list build and
+    // eight lanes in the mixed form's pair passes (same results): below these
+    // counts the thread-per-particle kernels leave SMs with too few warps to
+    // cover their loads.  Thread / lanes, us: 5,864 particles list 93 / 14,
+    // density 47 / 18, force 69 / 23; 22,040: 90 / 29, 47 / 31, 66 / 50; 39,464:
+    // 86 / 45, 45 / 42, 67 / 74; 64,280: 92 / 68, 49 / 61, 78 / 111; list of
+    // 85,544: 97 / 89, of 131,072: 91 / 131.
+    static constexpr int64_t kFewParticles = 32768, kFewForLists = 90112;
     // The FP64 form's pair passes take four lanes to a particle at every count:
     // its results may not depend on which impacts are resident, and the lanes'
     // partial sums do depend on their number.  One thread / 2 / 4 / 8 lanes, us:
@@ -2477,8 +2478,8 @@ public:
             k_list_thread<R, false, true><<<(unsigned)((N_ + bs - 1) / bs), bs, 0, st_>>>(view(), refresh);
             launched((const void*)k_list_thread<R, false, true>);
         } else if (N_ <= kFewForLists) {
-            k_list_group<R, 8><<<blocks_of(8 * N_), 256, 0, st_>>>(view(), refresh);
-            launched((const void*)k_list_group<R, 8>);
+            k_list_few<R><<<blocks_of(32 * N_), 256, 0, st_>>>(view(), refresh);
+            launched((const void*)k_list_few<R>);
         } else {
             k_list_thread<R, false, false><<<(unsigned)((N_ + bs - 1) / bs), bs, 0, st_>>>(view(), refresh);
             launched((const void*)k_list_thread<R, false, false>);

@@ -1121,11 +1121,11 @@ __device__ __forceinline__ void warp_walk_levels(const View<R>& v, const ImpactD
 // for a particle whose h outgrew the slack or whose list overflowed.
 //
 // Loop shape: the 32 particles of a warp are consecutive in sorted order, so
-// they sit in one or two cell columns and search nearly the same columns.  The
-// warp walks the union of its lanes' column boxes in a fixed order; each lane
-// takes the columns of its own box that meet its sphere, over the z-range of
-// its own chord, and the candidate loop runs to the longest chord of the warp
-// with the other lanes predicated off; a candidate costs one 16-byte load of
+// they sit in one or two cell columns and search nearly the same columns.
+// The warp walks the union of its lanes' column boxes in a fixed order (or each
+// lane its own box, see there); each lane takes the columns of its own box that
+// meet its sphere, over the z-range of its own chord, and the candidate loop
+// runs to the longest chord of the warp with the other lanes predicated off; a candidate costs one 16-byte load of
 // its list-frame record.  Every lane visits the same candidates in the same
 // order as traverse_sphere(), so the lists equal those of a per-thread
 // traversal entry for entry.
@@ -1210,31 +1210,49 @@ static __global__ void k_list_thread(View<R> v, int refresh) {
     hi0 = hi0 < 0 ? 0 : (hi0 > nf0 - 1 ? nf0 - 1 : hi0);
     lo1 = lo1 < 0 ? 0 : (lo1 > nf1 - 1 ? nf1 - 1 : lo1);
     hi1 = hi1 < 0 ? 0 : (hi1 > nf1 - 1 ? nf1 - 1 : hi1);
+    // The lanes walk the box around all their columns (the same column at a
+    // time: shared loads), or each its own box where that is much smaller: in a
+    // warp whose run of cells wraps to the next row the box around all spans
+    // the grid (131,072 particles: 121 -> 91 us, 1,048,576: 586 -> 529; own boxes
+    // alone: 97 and 567).
     const int ulo0 = __reduce_min_sync(full, act ? lo0 : INT_MAX), uhi0 = __reduce_max_sync(full, act ? hi0 : INT_MIN);
     const int ulo1 = __reduce_min_sync(full, act ? lo1 : INT_MAX), uhi1 = __reduce_max_sync(full, act ? hi1 : INT_MIN);
-    for (int ix = ulo0; ix <= uhi0; ix++) {
+    const int own = act ? (hi0 - lo0 + 1) * (hi1 - lo1 + 1) : 0;
+    int most = __reduce_max_sync(full, own);
+    const int around = (uhi0 - ulo0 + 1) * (uhi1 - ulo1 + 1);
+    const bool together = around <= most + most / 2;  // warp-uniform
+    const int blo0 = together ? ulo0 : lo0, blo1 = together ? ulo1 : lo1, bhi1 = together ? uhi1 : hi1;
+    if (together) most = around;
+    auto gap_x = [&](int ix) {
         const float xa = (float)(ix - c[0]) * w0 - pi.x;
-        float bx = xa > 0.0f ? xa : (xa + w0 < 0.0f ? -(xa + w0) : 0.0f);
-        if (ix == 0 || ix == nf0 - 1) bx = 0.0f;
-        const bool in_x = act && ix >= lo0 && ix <= hi0;
-        for (int iy = ulo1; iy <= uhi1; iy++) {
-            const float ya = (float)(iy - c[1]) * w1 - pi.y;
-            float by = ya > 0.0f ? ya : (ya + w1 < 0.0f ? -(ya + w1) : 0.0f);
-            if (iy == 0 || iy == nf1 - 1) by = 0.0f;
-            const float d2 = bx * bx + by * by;
-            int32_t s = 0, len = 0;
-            if (in_x && iy >= lo1 && iy <= hi1 && d2 < R2) {
-                const float q = R2 - d2;
-                const float hz = q * rsqrtf(q) * (1.0f + 1.0e-6f);  // hardware 1/sqrt (2 ulp), widened
-                int zl = c[2] + (int)floorf((pi.z - hz) * iw2 - kWiden);
-                int zh = c[2] + (int)floorf((pi.z + hz) * iw2 + kWiden);
-                zl = zl < 0 ? 0 : (zl > nf2 - 1 ? nf2 - 1 : zl);
-                zh = zh < 0 ? 0 : (zh > nf2 - 1 ? nf2 - 1 : zh);
-                const int64_t colbase = I.cell_base + ((int64_t)ix * nf1 + iy) * nf2;
-                s = v.cell_ptr[colbase + zl];
-                len = v.cell_ptr[colbase + zh + 1] - s;
-            }
-            run(s, len);
+        const float b = xa > 0.0f ? xa : (xa + w0 < 0.0f ? -(xa + w0) : 0.0f);
+        return ix == 0 || ix == nf0 - 1 ? 0.0f : b;
+    };
+    const int32_t* col = v.cell_ptr + I.cell_base + ((int64_t)blo0 * nf1 + blo1) * nf2;
+    const int64_t next_x = (int64_t)(nf1 - 1 - (bhi1 - blo1)) * nf2;
+    float bx = gap_x(blo0);
+    for (int n = 0, ix = blo0, iy = blo1; n < most; n++) {
+        const float ya = (float)(iy - c[1]) * w1 - pi.y;
+        float by = ya > 0.0f ? ya : (ya + w1 < 0.0f ? -(ya + w1) : 0.0f);
+        if (iy == 0 || iy == nf1 - 1) by = 0.0f;
+        const float d2 = bx * bx + by * by;
+        int32_t s = 0, len = 0;
+        if (act && ix >= lo0 && ix <= hi0 && iy >= lo1 && iy <= hi1 && d2 < R2) {
+            const float q = R2 - d2;
+            const float hz = q * rsqrtf(q) * (1.0f + 1.0e-6f);  // hardware 1/sqrt (2 ulp), widened
+            int zl = c[2] + (int)floorf((pi.z - hz) * iw2 - kWiden);
+            int zh = c[2] + (int)floorf((pi.z + hz) * iw2 + kWiden);
+            zl = zl < 0 ? 0 : (zl > nf2 - 1 ? nf2 - 1 : zl);
+            zh = zh < 0 ? 0 : (zh > nf2 - 1 ? nf2 - 1 : zh);
+            s = col[zl];
+            len = col[zh + 1] - s;
+        }
+        run(s, len);
+        col += nf2;
+        if (++iy > bhi1) {
+            iy = blo1;
+            col += next_x;
+            bx = gap_x(++ix);
         }
     }
     if (act) {
@@ -1244,27 +1262,20 @@ static __global__ void k_list_thread(View<R> v, int refresh) {
     }
 }
 
-// The list build with G lanes to a particle (non-periodic impacts on one grid):
-// a column's candidates are tested 2 G at a time and the hits appended in
-// candidate order by a ballot, so the lists are k_list_thread's entry for entry.
-// A run of few particles leaves that kernel's warps waiting on one candidate
-// pair after another; here the same waits cover eight times as many.
-template <class R, int G>
-static __global__ void __launch_bounds__(256) k_list_group(View<R> v, int refresh) {
+// The same lists with a warp to a particle, for runs of few particles, where
+// the chain of columns in the particles of the largest h decides: each lane
+// takes a column's chord, the chords' candidates are numbered by a prefix sum
+// and the warp tests 32 of them at a time, so the list comes out in the same
+// order.  5,864 particles: 92 us with a thread to a particle, 45 with eight
+// lanes that walked the columns together, 14 here.
+template <class R>
+static __global__ void __launch_bounds__(256) k_list_few(View<R> v, int refresh) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, g = lane & (G - 1), first = lane & ~(G - 1);
-    const int64_t k0 = gtid() / G;
-    const bool inb = k0 < v.n;
-    const int64_t k = inb ? k0 : v.n - 1;
-    const int ib = v.imp[k];
-    const ImpactD& I = v.imps[ib];
-    const bool wanted = I.mask && (!refresh || I.slack_flag);
-    const bool one_impact = __all_sync(full, ib == __shfl_sync(full, ib, 0));
-    if (!one_impact) {
-        if (inb && wanted && g == 0) list_one<R, false, false>(v, I, k);
-        return;
-    }
-    if (!wanted) return;  // warp-uniform: one impact
+    const int lane = threadIdx.x & 31;
+    const int64_t k = gtid() / 32;
+    if (k >= v.n) return;  // the whole warp
+    const ImpactD& I = v.imps[v.imp[k]];
+    if (!(I.mask && (!refresh || I.slack_flag))) return;
     const float4 pi = v.pf[k];
     const uint32_t ci = v.cpk[k];
     const float4 li = v.lf[k];
@@ -1277,9 +1288,9 @@ static __global__ void __launch_bounds__(256) k_list_group(View<R> v, int refres
     int cnt = 0;
     const int cap = v.cap;
     int32_t* out = v.nbr + 4 * k;  // entry t at out[nbr_slot(t, ls)]
-    const unsigned below = (1u << g) - 1u;
+    const unsigned below = (1u << lane) - 1u;
     auto take = [&](bool hit, int32_t j, float4 lj, float r2) {  // the whole warp
-        const unsigned hits = (__ballot_sync(full, hit) >> first) & ((1u << G) - 1u);
+        const unsigned hits = __ballot_sync(full, hit);
         if (hit) {
             const int at = cnt + __popc(hits & below);
             if (at < cap) out[nbr_slot(at, v.ls)] = j;
@@ -1305,42 +1316,56 @@ static __global__ void __launch_bounds__(256) k_list_group(View<R> v, int refres
     hi0 = hi0 < 0 ? 0 : (hi0 > nf0 - 1 ? nf0 - 1 : hi0);
     lo1 = lo1 < 0 ? 0 : (lo1 > nf1 - 1 ? nf1 - 1 : lo1);
     hi1 = hi1 < 0 ? 0 : (hi1 > nf1 - 1 ? nf1 - 1 : hi1);
-    const int ulo0 = __reduce_min_sync(full, inb ? lo0 : INT_MAX), uhi0 = __reduce_max_sync(full, inb ? hi0 : INT_MIN);
-    const int ulo1 = __reduce_min_sync(full, inb ? lo1 : INT_MAX), uhi1 = __reduce_max_sync(full, inb ? hi1 : INT_MIN);
-    for (int ix = ulo0; ix <= uhi0; ix++) {
+    const int ny = hi1 - lo1 + 1, ncol = (hi0 - lo0 + 1) * ny;
+    for (int base = 0; base < ncol; base += 32) {
+        const int q = base + lane;
+        const int ix = lo0 + q / ny, iy = lo1 + q % ny;
         const float xa = (float)(ix - c[0]) * w0 - pi.x;
         float bx = xa > 0.0f ? xa : (xa + w0 < 0.0f ? -(xa + w0) : 0.0f);
         if (ix == 0 || ix == nf0 - 1) bx = 0.0f;
-        const bool in_x = inb && ix >= lo0 && ix <= hi0;
-        for (int iy = ulo1; iy <= uhi1; iy++) {
-            const float ya = (float)(iy - c[1]) * w1 - pi.y;
-            float by = ya > 0.0f ? ya : (ya + w1 < 0.0f ? -(ya + w1) : 0.0f);
-            if (iy == 0 || iy == nf1 - 1) by = 0.0f;
-            const float d2 = bx * bx + by * by;
-            int32_t s = 0, len = 0;
-            if (in_x && iy >= lo1 && iy <= hi1 && d2 < R2) {
-                const float q = R2 - d2;
-                const float hz = q * rsqrtf(q) * (1.0f + 1.0e-6f);  // hardware 1/sqrt (2 ulp), widened
-                int zl = c[2] + (int)floorf((pi.z - hz) * iw2 - kWiden);
-                int zh = c[2] + (int)floorf((pi.z + hz) * iw2 + kWiden);
-                zl = zl < 0 ? 0 : (zl > nf2 - 1 ? nf2 - 1 : zl);
-                zh = zh < 0 ? 0 : (zh > nf2 - 1 ? nf2 - 1 : zh);
-                const int64_t colbase = I.cell_base + ((int64_t)ix * nf1 + iy) * nf2;
-                s = v.cell_ptr[colbase + zl];
-                len = v.cell_ptr[colbase + zh + 1] - s;
-            }
-            const int maxlen = __reduce_max_sync(full, len);
-            for (int t = 0; t < maxlen; t += 2 * G) {
-                const bool ok0 = t + g < len, ok1 = t + G + g < len;
-                const int32_t j0 = ok0 ? s + t + g : (int32_t)k, j1 = ok1 ? s + t + G + g : (int32_t)k;
-                const float4 l0 = v.lf[j0], l1 = v.lf[j1];
-                const float r20 = list_r2(li, l0), r21 = list_r2(li, l1);
-                take(ok0 && r20 < ri2, j0, l0, r20);
-                take(ok1 && r21 < ri2, j1, l1, r21);
-            }
+        const float ya = (float)(iy - c[1]) * w1 - pi.y;
+        float by = ya > 0.0f ? ya : (ya + w1 < 0.0f ? -(ya + w1) : 0.0f);
+        if (iy == 0 || iy == nf1 - 1) by = 0.0f;
+        const float d2 = bx * bx + by * by;
+        int32_t s = 0, len = 0;
+        if (q < ncol && d2 < R2) {
+            const float r = R2 - d2;
+            const float hz = r * rsqrtf(r) * (1.0f + 1.0e-6f);  // hardware 1/sqrt (2 ulp), widened
+            int zl = c[2] + (int)floorf((pi.z - hz) * iw2 - kWiden);
+            int zh = c[2] + (int)floorf((pi.z + hz) * iw2 + kWiden);
+            zl = zl < 0 ? 0 : (zl > nf2 - 1 ? nf2 - 1 : zl);
+            zh = zh < 0 ? 0 : (zh > nf2 - 1 ? nf2 - 1 : zh);
+            const int64_t colbase = I.cell_base + ((int64_t)ix * nf1 + iy) * nf2;
+            s = v.cell_ptr[colbase + zl];
+            len = v.cell_ptr[colbase + zh + 1] - s;
+        }
+        int end = len;  // candidates up to and with this chord's
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const int x = __shfl_up_sync(full, end, o);
+            if (lane >= o) end += x;
+        }
+        const int total = __shfl_sync(full, end, 31);
+        const int32_t at0 = s - (end - len);  // slot of candidate a of this chord: at0 + a
+        auto slot_of = [&](int a) {  // the first chord that ends past a
+            int r = 0;
+#pragma unroll
+            for (int o = 16; o > 0; o /= 2)
+                if (__shfl_sync(full, end, r + o - 1) <= a) r += o;
+            return a + __shfl_sync(full, at0, r);
+        };
+        for (int t = 0; t < total; t += 64) {
+            const int a0 = t + lane, a1 = a0 + 32;
+            const int32_t x0 = slot_of(a0), x1 = slot_of(a1);
+            const bool ok0 = a0 < total, ok1 = a1 < total;
+            const int32_t j0 = ok0 ? x0 : (int32_t)k, j1 = ok1 ? x1 : (int32_t)k;
+            const float4 l0 = v.lf[j0], l1 = v.lf[j1];
+            const float r20 = list_r2(li, l0), r21 = list_r2(li, l1);
+            take(ok0 && r20 < ri2, j0, l0, r20);
+            take(ok1 && r21 < ri2, j1, l1, r21);
         }
     }
-    if (inb && g == 0) {
+    if (lane == 0) {
         v.nbr_cnt[k] = cnt;
         v.hlist[k] = pi.w;
         if (cnt > cap) atomicMax(&v.flags[0], cnt);
