@@ -350,7 +350,7 @@ public:
         DSPH_CUDA(cudaEventCreateWithFlags(&out_ev_, cudaEventDisableTiming));
         DSPH_CUDA(cudaEventCreateWithFlags(&late_ev_, cudaEventDisableTiming));
         DSPH_CUDA(cudaMalloc(&mats_d_, sizeof(MatT<R>) * kMaxMaterials));
-        DSPH_CUDA(cudaMalloc(&flags_d_, sizeof(int32_t) * 4));
+        DSPH_CUDA(cudaMalloc(&flags_d_, sizeof(int32_t) * 8));
         DSPH_CUDA(cudaMalloc(&wait_err_d_, sizeof(int32_t)));
         DSPH_CUDA(cudaMemsetAsync(wait_err_d_, 0, sizeof(int32_t), st_));
         DSPH_CUDA(cudaMalloc(&ntask_, sizeof(int32_t)));
@@ -364,7 +364,7 @@ public:
             pageable_access_ = pa != 0;
         }
         DSPH_CUDA(cudaMallocHost(&flags_h_, sizeof(int32_t) * 4));
-        DSPH_CUDA(cudaMemsetAsync(flags_d_, 0, sizeof(int32_t) * 4, st_));
+        DSPH_CUDA(cudaMemsetAsync(flags_d_, 0, sizeof(int32_t) * 8, st_));
         for (int i = 0; i < 6; i++) DSPH_CUDA(cudaEventCreate(&ev_[i]));
         for (int i = 0; i < 5; i++) phase_ms_[i] = 0;
     }
@@ -2529,31 +2529,31 @@ public:
         const int nimp = (int)imp_.size();
         for (int round = 0; round < 4; round++) {
             cls(KC_GRID);
-            if (round > 0) launch_n_raw(k_ref_bins<R>, N_, view(), 0);
+            if (round > 0) launch_n_raw(k_ref_bins<R>, N_, view(), 0, round);
             cls(KC_DENSITY);
             if (iters > 0) {  // also reduces the new max h
                 constexpr int L = sizeof(R) == 8 ? kLanes64 : 1;
-                if (levels_active_) launch_n_raw(k_density<R, true, true, L>, L * N_, view(), iters);
-                else if (any_periodic()) launch_n_raw(k_density<R, false, true, L>, L * N_, view(), iters);
+                if (levels_active_) launch_n_raw(k_density<R, true, true, L>, L * N_, view(), iters, round);
+                else if (any_periodic()) launch_n_raw(k_density<R, false, true, L>, L * N_, view(), iters, round);
                 else if (few_particles()) {
-                    if constexpr (sizeof(R) == 4) launch_n_raw(k_density<R, false, false, 8>, 8 * N_, view(), iters);
+                    if constexpr (sizeof(R) == 4) launch_n_raw(k_density<R, false, false, 8>, 8 * N_, view(), iters, round);
                 }
-                else launch_n_raw(k_density<R, false, false, L>, L * N_, view(), iters);
+                else launch_n_raw(k_density<R, false, false, L>, L * N_, view(), iters, round);
             }
             else hmax_pass(1);
             cls(KC_GRID);
             if (host_sync) DSPH_CUDA(cudaMemsetAsync(flags_d_ + 1, 0, sizeof(int32_t), st_));
-            launch_small(k_round, nimp, flags_d_, round < 3 ? (int)kRoundNext : (int)kRoundFinal);
+            launch_small(k_round, nimp, flags_d_, round < 3 ? (int)kRoundNext : (int)kRoundFinal, round);
             if (host_sync && round < 3) {
                 DSPH_CUDA(cudaMemcpyAsync(flags_h_ + 1, flags_d_ + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st_));
                 DSPH_CUDA(cudaStreamSynchronize(st_));
                 if (!flags_h_[1]) {
-                    launch_small(k_round, nimp, flags_d_, (int)kRoundOnlyFinal);
+                    launch_small(k_round, nimp, flags_d_, (int)kRoundOnlyFinal, round);
                     break;
                 }
             }
         }
-        launch_n_raw(k_ref_bins<R>, N_, view(), host_sync || list_mode_ != 0 ? 0 : 1);
+        launch_n_raw(k_ref_bins<R>, N_, view(), host_sync || list_mode_ != 0 ? 0 : 1, 0);
     }
 
     // Reference grid and bins of the current h, outside the rounds.
@@ -2563,7 +2563,7 @@ public:
         launch_small(k_impact_begin_round, nimp);
         hmax_pass(0);
         launch_small(k_ref_grid, nimp);
-        launch_n_raw(k_ref_bins<R>, N_, view(), 0);
+        launch_n_raw(k_ref_bins<R>, N_, view(), 0, 0);
     }
 
     void forces(bool host_check) {
