@@ -52,7 +52,7 @@ UNIT = "particle-steps/s"
 # and k_force launch; its length (own + reverse entries per particle) is read
 # from the engine after the profiled steps.
 KERNEL_OF_CLASS = {"list_density": "k_list_thread", "density": "k_density", "force": "k_force",
-                   "eos": "k_eos", "damage": "k_damage", "finish": "k_finish"}
+                   "eos": "k_eos", "finish": "k_finish"}
 ALG_BYTES = {
     # k_list_thread: reads pf 16, cpk 4, refbin 8, imp 2; writes count 4 and 4 B per entry
     "list_density": (34, 4),
@@ -64,8 +64,8 @@ ALG_BYTES = {
     "force": (16 + 4 + 2 + 1 + 4 + 10 * 4 + 3 * 4 + 6 * 4 + 8 + (3 + 1 + 6 + 1) * 4, 4),
     # k_eos: reads rho, u 8, mat 1, D, S 6; writes P, cs, packed record 40
     "eos": (4 + 8 + 1 + 4 + 24 + 8 + 40, 0),
-    "damage": (4 + 4 + 4 + 8 + 4 + 4, 0),
-    "finish": (8 * 4 + 6 * 4 + 6 * 4, 0),
+    # k_finish: damage (28), then kick, u, S, yield and the CFL minimum
+    "finish": (4 + 4 + 4 + 8 + 4 + 4 + 8 * 4 + 6 * 4 + 6 * 4, 0),
 }
 # FP32 flops executed per list entry (per iteration for k_density), from the
 # ncu instruction counters of the mixed kernels (2 x FFMA + FADD + FMUL over

@@ -7,8 +7,8 @@
 //     sources, the yield surface, damage growth and the CFL speed in FP32 (the
 //     arithmetic of the reference's own GPU solver); the state and its
 //     Runge-Kutta updates, the fluidization update and dt in FP64.
-// The compute type R is the template parameter; state and right-hand side
-// are always FP64.  Literals are written as R(...) so that an
+// The compute type R is the template parameter; the state is always FP64, the
+// right-hand side stored in R.  Literals are written as R(...) so that an
 // FP32 instantiation never promotes to FP64.
 #pragma once
 
@@ -26,9 +26,9 @@ namespace deu {
 // as written; FP64 with the same IEEE results from the integer pipes
 // (fp64_int.cuh), because the FP64 kernels here wait on the FP64 pipe and
 // nothing else.  On the 96^3 impact (ncu) a face flux was 671 FP64
-// instructions and is 195 with these, the EOS's shared subexpressions and one
-// HLLC side per face; a face pass 1.14 -> 0.35 ms, a right-hand side 865 -> 266
-// instructions and 1.46 -> 0.61 ms, the step 11.1 -> 4.0 ms, same bits.
+// instructions and is 157 with these, the EOS's shared subexpressions and one
+// HLLC side per face; a face pass 1.14 -> 0.30 ms, a right-hand side 865 -> 194
+// instructions and 1.46 -> 0.39 ms, the step 11.1 -> 3.0 ms, same bits.
 template <class R>
 struct DivBy;  // a divisor used more than once
 template <>

@@ -263,7 +263,7 @@ int sph_debug_flaws(sph_ctx* ctx, int32_t impact, int64_t* ptr, double* eps, int
                     int64_t* total);
 
 /* ---- primitives on caller-owned device memory ------------------------------
- * Stable radix cell sort (the cell-list build of sph.hpp:147-162 as a
+ * Stable cell sort (the cell-list build of sph.hpp:147-162 as a
  * device primitive): keys[n] (device, uint32 cell ids in [0, ncells)) ->
  * perm[n] (device): particle indices ordered by (cell, index); cell_start
  * [ncells+1] (device): first sorted position of each cell, cell_start[ncells]
