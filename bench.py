@@ -666,7 +666,7 @@ def main():
                     help="mixed form: force-pass record staging (engine option force_staging)")
     ap.add_argument("--host-direct", type=int, default=None,
                     help="mixed form: 1 lets kernels reach host field buffers directly over the "
-                         "CPU-GPU link (engine option host_direct; default: device staging copies)")
+                         "CPU-GPU link (engine option host_direct; default: one launch to page-locked buffers, staging copies for others)")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-batch", action="store_true")
@@ -778,7 +778,7 @@ def main():
                "separate_calls": {"value": world * sc.n * args.steps / el_sep,
                                   "api": "sph_write_fields + sph_timestep + sph_step + sph_read_fields",
                                   "host_path": "direct (kernels over the CPU-GPU link)"
-                                  if ctx.get_option("host_direct") else "device staging copies"}}
+                                  if ctx.get_option("host_direct") else "one launch to page-locked buffers"}}
     ctx.close()
 
     # ---- plain FP64 form

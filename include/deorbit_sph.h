@@ -414,7 +414,9 @@ int sph_set_tuning(sph_ctx* ctx, int32_t block_threads, double cell_factor);
  * the force pass staged in shared memory; 0 off, 22 / 23 / 42 bulk copies of
  * 2 or 4 entries x 2 or 3 stages, 122 / 142 16-byte async copies),
  * "host_direct" (1: field reads and writes reach device-accessible host
- * buffers directly over the CPU-GPU link; 0: device staging copies);
+ * buffers directly over the CPU-GPU link, a launch per field, pageable memory
+ * where the device reads it; 0: page-locked buffers in one launch a call, others
+ * through device staging copies);
  * read-only "list_capacity" (entries per particle), "list_entries" (entries
  * of the current lists, own plus reverse), "device_bytes" (the context's
  * device allocations), "bytes_per_particle" (device bytes per particle of
