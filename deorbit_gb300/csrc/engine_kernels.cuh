@@ -1137,8 +1137,8 @@ __device__ __forceinline__ void warp_walk_levels(const View<R>& v, const ImpactD
 // The warp walks the union of its lanes' column boxes in a fixed order (or each
 // lane its own box, see there); each lane takes the columns of its own box that
 // meet its sphere, over the z-range of its own chord, and the candidate loop
-// runs to the longest chord of the warp with the other lanes predicated off; a candidate costs one 16-byte load of
-// its list-frame record.  Every lane visits the same candidates in the same
+// runs to the longest chord of the warp with the other lanes predicated off; a
+// candidate costs one 16-byte load of its list-frame record.  Every lane visits the same candidates in the same
 // order as traverse_sphere(), so the lists equal those of a per-thread
 // traversal entry for entry.
 //
@@ -1227,7 +1227,7 @@ static __global__ void k_list_thread(View<R> v, int refresh) {
     // time: shared loads), or each its own box where that is much smaller: in a
     // warp whose run of cells wraps to the next row the box around all spans
     // the grid (131,072 particles: 121 -> 91 us, 1,048,576: 586 -> 529; own boxes
-    // alone: 97 and 567).
+    // alone: 97 and 567; the line at 1.25 own boxes 94 and 541, at 2: 90 and 530).
     const int ulo0 = __reduce_min_sync(full, act ? lo0 : INT_MAX), uhi0 = __reduce_max_sync(full, act ? hi0 : INT_MIN);
     const int ulo1 = __reduce_min_sync(full, act ? lo1 : INT_MAX), uhi1 = __reduce_max_sync(full, act ? hi1 : INT_MIN);
     const int own = act ? (hi0 - lo0 + 1) * (hi1 - lo1 + 1) : 0;
